@@ -657,8 +657,11 @@ struct TcArgs {
     int BC;                          // chip columns per chunk of the chip operand (even)
     int MT;                          // MMA M: 64 or 128 surface columns
     int big;                         // 1: box sums before the products, chunks reuse their space
+                                     // 2: the same in stripes of VR surface rows
+    int VR;                          // k_corr_tc, big == 2: surface rows per box-sum stripe
     unsigned off_E, off_W, off_T, off_P, off_V, off_S1, off_S2, off_num, off_est, off_red;
-    int XV;                          // k_corr_tc2: row stride (words) of the column sums V1, V2
+    int XV;                          // row stride (words) of the column sums V1, V2 (k_corr_tc2;
+                                     // k_corr_tc with big == 2)
     int acc1_col;                    // stride between the accumulators (first column of the
                                      // second one)
     int issuers;                     // k_corr_tc: threads issuing the products, 2 or 4
@@ -1196,7 +1199,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_corr_tc(const TcArgs A) {
                     const int q = tq[u], x = tx[u];
                     const uint4 v = col16_finish(L[u]);
                     *reinterpret_cast<uint4*>(s_W + q * A.QS + x * 16) = v;
-                    if (x < XW && q >= qT) {
+                    if (A.big != 2 && x < XW && q >= qT) {
                         const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
                         for (int t = 0; t < 16; ++t)
@@ -1290,7 +1293,109 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_corr_tc(const TcArgs A) {
                 }
             }
         };
-        if (A.big) {
+        // The same sums in stripes of A.VR surface rows, for geometries whose column sums of every
+        // surface row do not fit beside the window (chips of 64 px and up with surfaces beyond
+        // 64 x 64). Column sums of a stripe straight from the 16-byte window blocks (no transposed
+        // copy): a thread per column, dp4a over the chip's rows for the stripe's first row, then a
+        // slide of four rows at a time. Row sums of a stripe as prefix sums, a warp per row: a
+        // difference of two prefixes is exact modulo 2^32 and the sums are below 2^32.
+        auto box_sums_striped = [&]() {
+            uint32_t* s_V2 = s_V1 + A.VR * A.XV;
+            for (int is = iA; is < nr; is += A.VR) {
+                const int ie = min(is + A.VR, nr);
+                for (int x = tid; x < XW; x += kTcThreads) {
+                    const uint8_t* col = s_W + x * 16;
+                    const int R0 = static_cast<int>(delta) + is, R1 = R0 + ch;
+                    uint32_t h1 = 0u, h2 = 0u;
+                    for (int q = R0 >> 4; 16 * q < R1; ++q) {
+                        const uint4 v = *reinterpret_cast<const uint4*>(col + q * A.QS);
+                        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+                        const int lo = R0 - 16 * q, hi = R1 - 16 * q;
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const int l = lo - 4 * u, h = hi - 4 * u;
+                            uint32_t m = l <= 0 ? 0xffffffffu : l >= 4 ? 0u : 0xffffffffu << (8 * l);
+                            m &= h >= 4 ? 0xffffffffu : h <= 0 ? 0u : (1u << (8 * h)) - 1u;
+                            const uint32_t wm = w[u] & m;
+                            h1 = __dp4a(wm, 0x01010101u, h1);
+                            h2 = __dp4a(wm, wm, h2);
+                        }
+                    }
+                    // The word of rows a .. a + 3 (a a multiple of 4, held to the staged blocks).
+                    auto word = [&](int a) {
+                        const int q = min(a >> 4, Q - 1);
+                        return *reinterpret_cast<const uint32_t*>(col + q * A.QS + (a & 12));
+                    };
+                    const uint32_t so = static_cast<uint32_t>(R0 & 3) * 8u;
+                    const uint32_t sn = static_cast<uint32_t>(R1 & 3) * 8u;
+                    int ao = R0 & ~3, an = R1 & ~3;
+                    uint32_t lo_o = word(ao), lo_n = word(an);
+                    uint32_t* v1 = s_V1 + x;
+                    uint32_t* v2 = s_V2 + x;
+                    for (int i = is; i < ie; i += 4) {
+                        ao += 4;
+                        an += 4;
+                        const uint32_t hi_o = word(ao), hi_n = word(an);
+                        const uint32_t wo = __funnelshift_r(lo_o, hi_o, so);
+                        const uint32_t wn = __funnelshift_r(lo_n, hi_n, sn);
+                        lo_o = hi_o;
+                        lo_n = hi_n;
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            if (i + u < ie) {
+                                *v1 = h1;
+                                *v2 = h2;
+                            }
+                            v1 += A.XV;
+                            v2 += A.XV;
+                            const uint32_t bo = (wo >> (8 * u)) & 255u, bn = (wn >> (8 * u)) & 255u;
+                            h1 += bn - bo;
+                            h2 += bn * bn - bo * bo;
+                        }
+                    }
+                }
+                __syncthreads();
+                for (int i = is + warp; i < ie; i += nwarps) {
+                    uint32_t* v1 = s_V1 + (i - is) * A.XV;
+                    uint32_t* v2 = s_V2 + (i - is) * A.XV;
+                    uint32_t c1 = 0u, c2 = 0u;
+                    for (int x0 = 0; x0 < XW; x0 += 128) {
+                        const int x = x0 + 4 * lane;
+                        uint4 a = make_uint4(0, 0, 0, 0), b = a;
+                        if (x < XW) {
+                            a = *reinterpret_cast<const uint4*>(v1 + x);
+                            b = *reinterpret_cast<const uint4*>(v2 + x);
+                        }
+                        a.y += a.x;
+                        a.z += a.y;
+                        a.w += a.z;
+                        b.y += b.x;
+                        b.z += b.y;
+                        b.w += b.z;
+                        const uint32_t t1 = warp_inclusive_scan(a.w), t2 = warp_inclusive_scan(b.w);
+                        const uint32_t p1 = t1 - a.w + c1, p2 = t2 - b.w + c2;
+                        if (x < XW) {
+                            *reinterpret_cast<uint4*>(v1 + x) =
+                                make_uint4(a.x + p1, a.y + p1, a.z + p1, a.w + p1);
+                            *reinterpret_cast<uint4*>(v2 + x) =
+                                make_uint4(b.x + p2, b.y + p2, b.z + p2, b.w + p2);
+                        }
+                        c1 += __shfl_sync(kFull, t1, 31);
+                        c2 += __shfl_sync(kFull, t2, 31);
+                    }
+                    __syncwarp();
+                    const int ri = ring(i);
+                    for (int j = lane; j < nc; j += 32) {
+                        s_S1[j * A.NRS + ri] = v1[j + cw - 1] - (j > 0 ? v1[j - 1] : 0u);
+                        s_S2[j * A.NRS + ri] = v2[j + cw - 1] - (j > 0 ? v2[j - 1] : 0u);
+                    }
+                }
+                __syncthreads();  // the next stripe, or the chip chunks, overwrite the sums
+            }
+        };
+        if (A.big == 2) {
+            box_sums_striped();
+        } else if (A.big) {
             if (warp < nwarps - NI) box_sums(kTcThreads - 32 * NI);
             __syncthreads();  // the chip chunks overwrite s_T and s_V
         }
@@ -1559,8 +1664,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_corr_tc(const TcArgs A) {
                 float bnd;
                 const float est = tc_estimate(d, s_S1[os], s_S2[os], nnf, csf, kk, kk7, A.measure, &bnd);
                 s_num[o] = d;
-                s_est[o] = est;
-                s_est[o + A.NCM * A.NRS] = bnd;
+                s_est[o] = est + bnd;
                 lmax = fmaxf(lmax, est - bnd);
             }
         };
@@ -1644,8 +1748,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_corr_tc(const TcArgs A) {
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     if (in[u]) {
-                        s_est[o[u]] = ev[u];
-                        s_est[o[u] + A.NCM * A.NRS] = bv[u];
+                        s_est[o[u]] = ev[u] + bv[u];
                         lmax = fmaxf(lmax, ev[u] - bv[u]);
                     }
                 }
@@ -1669,7 +1772,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_corr_tc(const TcArgs A) {
             for (int e = tid; e < ne; e += 4 * kTcThreads) {
                 int o[4], ii[4], jj[4];
                 bool in[4];
-                float est[4], bnd[4];
+                float upb[4];
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     in[u] = e + u * kTcThreads < ne;
@@ -1679,13 +1782,10 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_corr_tc(const TcArgs A) {
                     fstep(fi, fj);
                 }
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    est[u] = in[u] ? s_est[o[u]] : 0.0f;
-                    bnd[u] = in[u] ? s_est[o[u] + A.NCM * A.NRS] : 0.0f;
-                }
+                for (int u = 0; u < 4; ++u) upb[u] = in[u] ? s_est[o[u]] : 0.0f;
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    if (!in[u] || (!(est[u] + bnd[u] >= M) && !isnan(est[u]))) continue;
+                    if (!in[u] || (!(upb[u] >= M) && !isnan(upb[u]))) continue;
                     const int os = jj[u] * A.NRS + ring(ii[u]);
                     const float v =
                         tc_exact(s_num[o[u]], s_S1[os], s_S2[os], mean, nn, cnorm, A.measure);
@@ -3783,7 +3883,7 @@ size_t tmem_smem_floor(uint32_t cols, size_t static_smem) {
 struct TcPlan {
     int NB, QM, QS, PS, PC, XS, XT, NRS, NRM, NCM, CHM, CWM, BC, big, MT;
     unsigned off_E, off_W, off_T, off_P, off_V, off_S1, off_S2, off_num, off_est, off_red;
-    int XV = 0, acc1_col = 0, issuers = 2;
+    int XV = 0, VR = 0, acc1_col = 0, issuers = 2;
     uint32_t tmem_cols;
     size_t smem;
 };
@@ -3945,7 +4045,8 @@ void four_issuers(TcPlan* P) {
 // fit the kernel (surface wider than 64 columns, more than 256 rows, chips taller than 226).
 // The whole chip operand and separate box-sum buffers when they fit ("overlap": the box sums
 // run beside the products); otherwise the box sums first and the chip operand in chunks of BC
-// columns in the space they used.
+// columns in the space they used; where even that space is too small for the column sums of every
+// surface row (chips of 64 px and up with surfaces beyond 64 x 64), the box sums in stripes.
 bool plan_corr_tc(const PassGeometry& g, size_t smem_cap, TcPlan* P) {
     const int ch = static_cast<int>(g.max_ch), cw = static_cast<int>(g.max_cw);
     const int nr = static_cast<int>(g.max_nr), nc = static_cast<int>(g.max_nc);
@@ -3981,7 +4082,7 @@ bool plan_corr_tc(const PassGeometry& g, size_t smem_cap, TcPlan* P) {
     const size_t Vb = a16(2ull * nr * (cw + nc - 1) * 4);
     const size_t nbytes = a16(static_cast<size_t>(nc) * P->NRS * 4);
     const size_t red = 3 * 32 * 8;
-    // Overlap layout: [E][W][T][P][V | num, est, bound][S1][S2][red].
+    // Overlap layout: [E][W][T][P][V | num, upper bounds][S1][S2][red].
     {
         size_t off = 0;
         P->off_E = 0;
@@ -3995,7 +4096,7 @@ bool plan_corr_tc(const PassGeometry& g, size_t smem_cap, TcPlan* P) {
         P->off_V = static_cast<unsigned>(off);
         P->off_num = P->off_V;
         P->off_est = static_cast<unsigned>(off + nbytes);
-        off += std::max(Vb, 3 * nbytes);
+        off += std::max(Vb, 2 * nbytes);
         P->off_S1 = static_cast<unsigned>(off);
         off += nbytes;
         P->off_S2 = static_cast<unsigned>(off);
@@ -4010,31 +4111,68 @@ bool plan_corr_tc(const PassGeometry& g, size_t smem_cap, TcPlan* P) {
             return true;
         }
     }
+    // The chip operand in chunks of at most `avail` bytes: as few as fit, of even, equal widths.
+    auto chunk = [&](size_t avail) {
+        const int most = static_cast<int>(std::min<size_t>(cw, avail / P->PS)) & ~1;
+        if (most < 2) return 0;
+        const int n = (cw + most - 1) / most;
+        return std::min(most, round_up((cw + n - 1) / n, 2));
+    };
     // Chunked layout: [W][P][S1][S2][red][zone], the zone holding T and V for the box sums,
-    // then the chunks of the chip operand, then num, estimates and bounds.
+    // then the chunks of the chip operand, then num and the upper bounds.
+    {
+        size_t off = 0;
+        P->off_W = 0;
+        off += Wb;
+        P->off_P = static_cast<unsigned>(off);
+        off += Pb;
+        P->off_S1 = static_cast<unsigned>(off);
+        off += nbytes;
+        P->off_S2 = static_cast<unsigned>(off);
+        off += nbytes;
+        P->off_red = static_cast<unsigned>(off);
+        off += red;
+        off = a16(off);
+        const size_t zone_min = std::max(Tb + Vb, 2 * nbytes);
+        if (off + std::max(zone_min, 2 * static_cast<size_t>(P->PS)) <= smem_cap) {
+            const int bc = chunk(smem_cap - off);
+            if (bc < 2) return false;
+            P->BC = bc;
+            P->big = 1;
+            P->off_E = P->off_T = P->off_num = static_cast<unsigned>(off);
+            P->off_V = static_cast<unsigned>(off + Tb);
+            P->off_est = static_cast<unsigned>(off + nbytes);
+            P->smem = off + std::max(zone_min, static_cast<size_t>(bc) * P->PS);
+            four_issuers(P);
+            return true;
+        }
+    }
+    // Striped layout: [S1][S2][red][P][W][zone], the zone holding V of a stripe of 16 or more
+    // surface rows, then the chunks of the chip operand; num and the upper bounds take W and the
+    // zone once the products are done (P keeps its zero padding between points).
     size_t off = 0;
-    P->off_W = 0;
-    off += Wb;
-    P->off_P = static_cast<unsigned>(off);
-    off += Pb;
-    P->off_S1 = static_cast<unsigned>(off);
+    P->off_S1 = 0;
     off += nbytes;
     P->off_S2 = static_cast<unsigned>(off);
     off += nbytes;
     P->off_red = static_cast<unsigned>(off);
-    off += red;
-    off = a16(off);
-    const size_t zone_min = std::max(Tb + Vb, 3 * nbytes);
-    if (off + std::max(zone_min, 2 * static_cast<size_t>(P->PS)) > smem_cap) return false;
-    const size_t avail = smem_cap - off;
-    int bc = static_cast<int>(std::min<size_t>(cw, avail / P->PS)) & ~1;
+    off = a16(off + red);
+    P->off_P = static_cast<unsigned>(off);
+    off += Pb;
+    P->off_W = P->off_num = static_cast<unsigned>(off);
+    P->off_est = static_cast<unsigned>(off + nbytes);
+    const size_t num_end = off + 2 * nbytes;
+    off += Wb;
+    P->XV = round_up(cw + nc - 1, 4);
+    const size_t row = 2 * static_cast<size_t>(P->XV) * 4;
+    if (std::max(num_end, off + std::max<size_t>(16 * row, 2 * P->PS)) > smem_cap) return false;
+    const int bc = chunk(smem_cap - off);
     if (bc < 2) return false;
     P->BC = bc;
-    P->big = 1;
-    P->off_E = P->off_T = P->off_num = static_cast<unsigned>(off);
-    P->off_V = static_cast<unsigned>(off + Tb);
-    P->off_est = static_cast<unsigned>(off + nbytes);
-    P->smem = off + std::max(zone_min, static_cast<size_t>(bc) * P->PS);
+    P->big = 2;
+    P->VR = std::min(round_up(nr, 16), static_cast<int>((smem_cap - off) / row) & ~15);
+    P->off_E = P->off_T = P->off_V = static_cast<unsigned>(off);
+    P->smem = std::max(num_end, off + std::max(P->VR * row, static_cast<size_t>(bc) * P->PS));
     four_issuers(P);
     return true;
 }
@@ -4417,6 +4555,7 @@ cudaError_t launch_track_impl(int dtype, const void* ref, const void* sec, const
         B.CWM = TP.CWM;
         B.BC = TP.BC;
         B.big = TP.big;
+        B.VR = TP.VR;
         B.MT = TP.MT;
         B.off_E = TP.off_E;
         B.off_W = TP.off_W;
