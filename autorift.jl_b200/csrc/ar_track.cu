@@ -111,14 +111,33 @@ __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v)
     return v;
 }
 
+// Largest value of a warp (no lane NaN): floats as ordered integers, one reduction instruction.
+__device__ __forceinline__ float warp_max(float v) {
+    int i = __float_as_int(v);
+    i ^= (i >> 31) & 0x7fffffff;
+    i = __reduce_max_sync(kFull, i);
+    return __int_as_float(i ^ ((i >> 31) & 0x7fffffff));
+}
+
+// A barrier over the block, or (MAIN) over its first 256 threads (k_corr_tc2's main warps).
+template <bool MAIN>
+__device__ __forceinline__ void block_sync() {
+    if constexpr (MAIN) {
+        asm volatile("bar.sync 2, 256;" ::: "memory");
+    } else {
+        __syncthreads();
+    }
+}
+
 // Block-wide max; every thread gets the result. `red` holds >= 32 entries.
+template <bool MAIN = false>
 __device__ unsigned long long block_max_u64(unsigned long long v, unsigned long long* red) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nw = (blockDim.x + 31) >> 5;
+    const int nw = MAIN ? 8 : (blockDim.x + 31) >> 5;
     v = warp_max_u64(v);
-    __syncthreads();
+    block_sync<MAIN>();
     if (lane == 0) red[warp] = v;
-    __syncthreads();
+    block_sync<MAIN>();
     unsigned long long r = lane < nw ? red[lane] : 0ull;
     r = warp_max_u64(r);
     return r;
@@ -131,18 +150,18 @@ __device__ __forceinline__ double warp_sum_f64(double v) {
 }
 
 // Block-wide sum of up to three doubles; every thread gets the results.
-template <int N>
+template <int N, bool MAIN = false>
 __device__ void block_sum_f64(double (&v)[N], double* red) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nw = (blockDim.x + 31) >> 5;
+    const int nw = MAIN ? 8 : (blockDim.x + 31) >> 5;
 #pragma unroll
     for (int q = 0; q < N; ++q) v[q] = warp_sum_f64(v[q]);
-    __syncthreads();
+    block_sync<MAIN>();
     if (lane == 0) {
 #pragma unroll
         for (int q = 0; q < N; ++q) red[q * 32 + warp] = v[q];
     }
-    __syncthreads();
+    block_sync<MAIN>();
 #pragma unroll
     for (int q = 0; q < N; ++q) {
         double r = lane < nw ? red[q * 32 + lane] : 0.0;
@@ -641,7 +660,7 @@ __global__ void __launch_bounds__(kCorrThreads, 2) k_corr(const CorrArgs A) {
 // the largest estimate, and the patch, get the reference's exact FP64 normalisation.
 
 constexpr int kTcThreads = 256;
-constexpr int kTc2Issuers = 3;  // k_corr_tc2: threads issuing a point's products
+constexpr int kTc2Threads = 320;  // k_corr_tc2: eight main warps, a fetch warp, a patch warp
 constexpr int kPadL = 32;            // zero bytes before each staged chip column
 constexpr uint32_t kTcWaitPolls = 1u << 22;
 
@@ -660,6 +679,7 @@ struct TcArgs {
                                      // 2: the same in stripes of VR surface rows
     int VR;                          // k_corr_tc, big == 2: surface rows per box-sum stripe
     unsigned off_E, off_W, off_T, off_P, off_V, off_S1, off_S2, off_num, off_est, off_red;
+    unsigned off_L, off_rawW, off_rawC;  // k_corr_tc2
     int XV;                          // row stride (words) of the column sums V1, V2 (k_corr_tc2;
                                      // k_corr_tc with big == 2)
     int acc1_col;                    // stride between the accumulators (first column of the
@@ -853,6 +873,7 @@ __device__ __forceinline__ uint4 col16_finish(const Col16& L) {
 // while K stays below 2^53 -- guaranteed when (its terms) x (255 nn)^2 is: then the partial is
 // that integer scaled by 1/nn^2, the double the FP64 loop produces. Other areas take the FP64
 // loop over the staged chip.
+template <bool MAIN = false>
 __device__ __forceinline__ void staged_chip_stats(const uint8_t* s_P, int PC, int ch, int cw, int tid,
                                                   int bd, double* s_red, double* csum, double* mean,
                                                   double* sq) {
@@ -892,7 +913,7 @@ __device__ __forceinline__ void staged_chip_stats(const uint8_t* s_P, int PC, in
         }
     }
     double st[1] = {static_cast<double>(P)};
-    block_sum_f64<1>(st, s_red);
+    block_sum_f64<1, MAIN>(st, s_red);
     *csum = st[0];
     const int nn = ch * cw;
     const double mn = __ddiv_rn(st[0], static_cast<double>(nn));
@@ -917,7 +938,7 @@ __device__ __forceinline__ void staged_chip_stats(const uint8_t* s_P, int PC, in
             step(a, b);
         }
     }
-    block_sum_f64<1>(acc2, s_red);
+    block_sum_f64<1, MAIN>(acc2, s_red);
     *sq = acc2[0];
 }
 
@@ -1915,372 +1936,512 @@ __device__ __forceinline__ void pt_geometry(const TcArgs& A, int64_t k, PtGeo& g
     g.ok = 1;
 }
 
-__global__ void __launch_bounds__(kTcThreads, 2) k_corr_tc2(const TcArgs A) {
+// One CTA is eight main warps, a fetch warp and a patch warp, two CTAs to an SM. The fetch warp reads the points ahead (geometry of 32 points at a time, one per lane)
+// and copies the next point's window, chip and mask chunks into shared memory with cp.async
+// while the current point's peak is found. The patch warp turns the 5 x 5 numerators of a finished
+// point into the exact FP64 patch. So the main warps see neither global latency nor the FP64
+// chains: they stage the operands, issue the products (lane 0 of the last A.issuers warps, each
+// into its own accumulator), sum the boxes beside them, and find the peak. They meet the fetch warp
+// at two mbarriers (`full`: a point's geometry and chunks are in place, `free`: the chunks and the
+// column sums that share their space are read) and the patch warp at a barrier before the
+// products and at `out` (the patch is handed over); the waits on mbarriers are bounded, and
+// whoever gives up still takes the others to their next barrier.
+//
+// Bound: instruction issue of the CUDA-core work around the products (15 k warp instructions a point
+// at chip 32 / radius 25; 51 % issue utilisation with two CTAs of 96 registers a thread, tensor
+// pipe 20 %). Measured on that pass, 251 001 points: 9.96 ms before the extra warps, with three
+// issuing warps that also made the chip's FP64 statistics and the next geometry, patches in a main
+// warp, a bound computed with every estimate and column sums started afresh for every point; 6.99 ms
+// now. Three CTAs of 64 registers (two accumulators, no ring of reciprocal roots) measured 7.83 ms,
+// products issued by four lanes of the patch warp 7.60 ms, by two lanes each of the fetch and patch
+// warps 8 % above this.
+struct Tc2Pt {
+    long long k;  // point, or -1: no more points
+    long long chip_r, chip_c, win_r, win_c;
+    int ch, cw, nr, nc;
+    int raw;       // bit 0: the window's chunks are in s_rawW, bit 1: the chip's and mask's in s_rawC
+};
+
+// A finished point, for the patch warp.
+struct Tc2Out {
+    long long k;
+    int nr, nc, nn;
+    int kind;      // 1: the peak alone, 2: the patch
+    int pi, pj;    // the peak (kind 1) or the patch's first row and column
+    uint32_t cs, c2;      // chip sums (power-of-two areas)
+    double mean, sq, csum;  // chip statistics (other areas)
+    uint32_t D[25], s2[25];
+    float s1[25];
+};
+
+__device__ __forceinline__ const uint8_t* align16(const uint8_t* p) {
+    return reinterpret_cast<const uint8_t*>(reinterpret_cast<uintptr_t>(p) & ~uintptr_t(15));
+}
+__device__ __forceinline__ uint32_t tc2_low(const uint8_t* p) {
+    return static_cast<uint32_t>(reinterpret_cast<uintptr_t>(p));
+}
+
+// Power-of-two chip areas up to 4096 pixels: every term of the reference's FP64 chip sums is exact,
+// so mean = sum / nn and sq = (nn sum(C^2) - sum(C)^2) / nn.
+__device__ __forceinline__ bool tc2_exact_sums(int nn) { return (nn & (nn - 1)) == 0 && nn <= 4096; }
+__device__ __forceinline__ void tc2_chip_stats(int nn, uint32_t cs, uint32_t c2, double* mean, double* sq) {
+    const unsigned long long d =
+        static_cast<unsigned long long>(nn) * c2 - static_cast<unsigned long long>(cs) * cs;
+    *mean = __ddiv_rn(static_cast<double>(cs), static_cast<double>(nn));
+    *sq = __ddiv_rn(static_cast<double>(d), static_cast<double>(nn));
+}
+
+__device__ __forceinline__ void bar_main() { block_sync<true>(); }
+// The main warps and the patch warp.
+__device__ __forceinline__ void bar_products() { asm volatile("bar.sync 3, 288;" ::: "memory"); }
+__device__ __forceinline__ bool bar_main_or(bool v) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "bar.red.or.pred q, 2, 256, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t"
+        "}\n"
+        : "=r"(r)
+        : "r"(static_cast<uint32_t>(v))
+        : "memory");
+    return r != 0u;
+}
+
+// The rare paths as calls, so that their code stays out of the point loop: sixteen image rows at
+// the image's border, and an exact value.
+__device__ __noinline__ uint4 tc2_border(const uint8_t* img, const uint8_t* img_end, int64_t nrows,
+                                         int64_t ncols, int64_t c, int64_t r0) {
+    return col16_finish(col16_issue(img, img_end, nrows, ncols, c, r0));
+}
+__device__ __noinline__ float tc2_exact(uint32_t D, float s1, uint32_t s2, double mean, double nn,
+                                        double cnorm, int measure) {
+    return tc_exact(D, __float2uint_rn(s1), s2, mean, nn, cnorm, measure);
+}
+
+__global__ void __launch_bounds__(kTc2Threads, 2) k_corr_tc2(const TcArgs A) {
     extern __shared__ __align__(1024) unsigned char smem_tc[];
-    __shared__ uint64_t s_mbar;
+    __shared__ uint64_t s_mbar, s_full, s_free, s_outb[2];
     __shared__ uint32_t s_taddr;
-    __shared__ int s_slot;
-    __shared__ int s_ncand;
-    __shared__ uint32_t s_pd[25];
-    __shared__ float s_fmax[kTcThreads / 32];
-    __shared__ unsigned long long s_isum[2][2];
-    __shared__ PtGeo s_geo[2];  // by iteration parity: a point's geometry, computed ahead
+    __shared__ int s_fail, s_more[2];  // s_more, by result slot: a measured point, or the end
+    __shared__ float s_bu;
+    __shared__ float s_top[8], s_sec[8];
+    __shared__ int s_at[8];
+    __shared__ uint32_t s_isum[2][2];
+    __shared__ Tc2Pt s_pt[2];   // by the parity of the point's number in this CTA
+    __shared__ Tc2Out s_out[2];
     uint8_t* s_E = smem_tc + A.off_E;
     uint8_t* s_W = smem_tc + A.off_W;
     uint8_t* s_P = smem_tc + A.off_P;
     uint32_t* s_V1 = reinterpret_cast<uint32_t*>(smem_tc + A.off_V);
-    uint32_t* s_V2 = s_V1 + A.NRM * A.XV + 16;
-    uint32_t* s_S1 = reinterpret_cast<uint32_t*>(smem_tc + A.off_S1);
+    uint32_t* s_V2 = s_V1 + A.VR * A.XV + 16;
+    uint32_t* s_L1 = reinterpret_cast<uint32_t*>(smem_tc + A.off_L);
+    uint32_t* s_L2 = s_L1 + A.XV;
+    uint4* s_rawW = reinterpret_cast<uint4*>(smem_tc + A.off_rawW);
+    uint4* s_rawC = reinterpret_cast<uint4*>(smem_tc + A.off_rawC);
+    float* s_S1 = reinterpret_cast<float*>(smem_tc + A.off_S1);
     uint32_t* s_S2 = reinterpret_cast<uint32_t*>(smem_tc + A.off_S2);
+    float* s_R = reinterpret_cast<float*>(smem_tc + A.off_est);
     uint32_t* s_num = reinterpret_cast<uint32_t*>(smem_tc + A.off_num);
-    uint32_t* s_cI = reinterpret_cast<uint32_t*>(smem_tc + A.off_est);
     double* s_red = reinterpret_cast<double*>(smem_tc + A.off_red);
 
-    const int tid = threadIdx.x, bd = blockDim.x;
-    const int lane = tid & 31, warp = tid >> 5, nwarps = bd >> 5;
+    const int tid = threadIdx.x;
+    const int lane = tid & 31, warp = tid >> 5;
     const uint8_t* ref_end = A.ref + A.nrows * A.ncols;
+    const uint8_t* sec_end = A.sec + A.nrows * A.ncols;
+    const uint8_t* valid_end = A.valid + A.nrows * A.ncols;
 
-    if (tid < 2) s_geo[tid].k = -1;
     if (warp == 0) {
         tc::tmem_alloc(&s_taddr, A.tmem_cols);
         tc::tmem_relinquish();
     }
     if (tid == 0) {
-        tc::mbar_init(&s_mbar, kTc2Issuers);  // one commit per issuing thread
+        tc::mbar_init(&s_mbar, A.issuers);  // one commit per issuing thread
+        tc::mbar_init(&s_full, 1);
+        tc::mbar_init(&s_free, 1);
+        // One arrival per main warp. One per slot: a point's arrivals may come before the product
+        // warp has seen its predecessor's.
+        tc::mbar_init(&s_outb[0], 8);
+        tc::mbar_init(&s_outb[1], 8);
         tc::fence_mbar_init();
+        s_fail = 0;
     }
+    if (tid < 4) s_isum[tid >> 1][tid & 1] = 0u;
+    for (int e = tid; e < A.CWM * A.PC; e += kTc2Threads) s_P[e] = 0;
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t taddr = s_taddr;
     const uint32_t acc1 = static_cast<uint32_t>(A.acc1_col);  // stride between accumulators
-    uint32_t phase = 0;
-    bool failed = false;
-    if (tid < 4) s_isum[tid >> 1][tid & 1] = 0ull;
-    for (int e = tid; e < A.CWM * A.PC; e += bd) s_P[e] = 0;
-    int iter = 0;
-    int dirty_ch = 0;
-    TC_PHASE_INIT
-#ifdef AR_TC_PHASES
-    unsigned long long tmi_issue = 0, tmi_done = 0;
-#endif
+    // Clears the accumulator columns [32 half, 32 half + 32) of this warp's lane quarter.
+    auto clear_acc = [&]() {
+        uint32_t zero[16];
+#pragma unroll
+        for (int v = 0; v < 16; ++v) zero[v] = 0u;
+        const uint32_t lq = taddr + (static_cast<uint32_t>(32 * (warp & 3)) << 16) +
+                            static_cast<uint32_t>(32 * (warp >> 2));
+        if (32u * static_cast<uint32_t>(warp >> 2) < acc1) {
+            for (int v = 0; v < A.issuers; ++v) {
+                tc::tmem_st16(lq + static_cast<uint32_t>(v) * acc1, zero);
+                tc::tmem_st16(lq + static_cast<uint32_t>(v) * acc1 + 16u, zero);
+            }
+        }
+    };
 
     // Each CTA takes a contiguous run of points: consecutive points of a grid column have the
     // same window columns one grid step lower, so most of their box sums carry over.
     const int64_t per = (A.pts.n + gridDim.x - 1) / gridDim.x;
     const int64_t kbeg = static_cast<int64_t>(blockIdx.x) * per;
     const int64_t kend = min(A.pts.n, kbeg + per);
-    // The point whose box sums s_S1 / s_S2 hold (held = false: none).
+
+    if (warp == 8) {
+        // ------------------------------------------------------------------------------ helper
+        int64_t kb = kbeg - 32;   // the lanes hold the geometry of points kb .. kb + 31
+        unsigned okm = 0u;        // of those, the ones still to be correlated
+        PtGeo mine{};
+        // The next point to correlate and its chunks' copies, into slot `b`.
+        auto fetch = [&](int b) {
+            while (okm == 0u && kb + 32 < kend) {
+                kb += 32;
+                mine.ok = 0;
+                if (kb + lane < kend) pt_geometry(A, kb + lane, mine);
+                okm = __ballot_sync(kFull, mine.ok);
+            }
+            if (okm == 0u) {
+                if (lane == 0) s_pt[b].k = -1;
+                return false;
+            }
+            const int src = __ffs(okm) - 1;
+            okm &= okm - 1u;
+            const long long chip_r = __shfl_sync(kFull, mine.chip_r, src);
+            const long long chip_c = __shfl_sync(kFull, mine.chip_c, src);
+            const long long win_r = __shfl_sync(kFull, mine.win_r, src);
+            const long long win_c = __shfl_sync(kFull, mine.win_c, src);
+            const int ch = __shfl_sync(kFull, mine.ch, src), cw = __shfl_sync(kFull, mine.cw, src);
+            const int nr = __shfl_sync(kFull, mine.nr, src), nc = __shfl_sync(kFull, mine.nc, src);
+            const int XW = cw + nc - 1, RQ = (ch + nr - 1 + 15) / 16 + 1, RC = (ch + 15) / 16 + 1;
+            // Chunks: the aligned 16-byte blocks that hold a column's rows, when every row lies in
+            // the image and every block in the array.
+            const uint8_t* w0 = A.ref + win_c * A.nrows + win_r;
+            const uint8_t* w1 = w0 + static_cast<int64_t>(XW - 1) * A.nrows;
+            const bool rw = win_r >= 0 && win_r + 16 * (RQ - 1) <= A.nrows && win_c >= 0 &&
+                            win_c + XW <= A.ncols && align16(w0) >= A.ref &&
+                            align16(w1) + 16 * RQ <= ref_end;
+            const int64_t co = chip_c * A.nrows + chip_r, ce = co + static_cast<int64_t>(cw - 1) * A.nrows;
+            const bool rc = chip_r >= 0 && chip_r + ch <= A.nrows && chip_c >= 0 &&
+                            chip_c + cw <= A.ncols && align16(A.sec + co) >= A.sec &&
+                            align16(A.sec + ce) + 16 * RC <= sec_end &&
+                            align16(A.valid + co) >= A.valid &&
+                            align16(A.valid + ce) + 16 * RC <= valid_end;
+            if (lane == 0) {
+                Tc2Pt& p = s_pt[b];
+                p.k = kb + src;
+                p.chip_r = chip_r;
+                p.chip_c = chip_c;
+                p.win_r = win_r;
+                p.win_c = win_c;
+                p.ch = ch;
+                p.cw = cw;
+                p.nr = nr;
+                p.nc = nc;
+                p.raw = (rw ? 1 : 0) | (rc ? 2 : 0);
+            }
+            if (rc) {
+                const uint32_t inv = (65536u + static_cast<uint32_t>(RC) - 1u) / static_cast<uint32_t>(RC);
+                for (int t = lane; t < cw * RC; t += 32) {
+                    const int b2 = static_cast<int>((static_cast<uint32_t>(t) * inv) >> 16), kc = t - b2 * RC;
+                    const int64_t o = co + static_cast<int64_t>(b2) * A.nrows;
+                    tc::cp_async16(s_rawC + kc * cw + b2, align16(A.sec + o) + 16 * kc);
+                    tc::cp_async16(s_rawC + (RC + kc) * cw + b2, align16(A.valid + o) + 16 * kc);
+                }
+            }
+            if (rw) {
+                const uint32_t inv = (65536u + static_cast<uint32_t>(RQ) - 1u) / static_cast<uint32_t>(RQ);
+                for (int t = lane; t < XW * RQ; t += 32) {
+                    const int x = static_cast<int>((static_cast<uint32_t>(t) * inv) >> 16), kq = t - x * RQ;
+                    tc::cp_async16(s_rawW + kq * XW + x,
+                                   align16(w0 + static_cast<int64_t>(x) * A.nrows) + 16 * kq);
+                }
+            }
+            tc::cp_async_commit();
+            return true;
+        };
+        auto publish = [&]() {
+            tc::cp_async_wait_all();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&s_full);
+        };
+        bool more = fetch(0);
+        publish();
+        for (uint32_t b = 1, ph = 0; more; b ^= 1u, ph ^= 1u) {
+            if (!__all_sync(kFull, tc::mbar_wait(&s_free, ph, kTcWaitPolls))) break;
+            more = fetch(static_cast<int>(b));
+            publish();
+        }
+    } else if (warp == 9) {
+        // ----------------------------------------------------------------------------- patches
+        uint32_t ph = 0;  // the phase of `out`: each slot's own, the same for two points
+        for (int b = 0;; b ^= 1) {
+            bar_products();
+            if (!s_more[b]) break;
+            const Tc2Out& o = s_out[b];
+            const int nnl = o.nn;
+            const bool pow2 = tc2_exact_sums(nnl);
+            const double nn = static_cast<double>(nnl);
+            double mean = o.mean, sq = o.sq;
+            if (pow2) tc2_chip_stats(nnl, o.cs, o.c2, &mean, &sq);
+            const double cnorm = __dsqrt_rn(sq);
+            if (!__all_sync(kFull, tc::mbar_wait(&s_outb[b], ph, kTcWaitPolls))) {
+                // The main warps left, or will: wait for the barrier that ends them.
+                if (lane == 0) s_fail = 1;
+                __syncwarp();
+                ph ^= static_cast<uint32_t>(b);
+                continue;
+            }
+            ph ^= static_cast<uint32_t>(b);
+            const bool patch = o.kind == 2;
+            int slot = 0;
+            if (patch && lane == 0) slot = atomicAdd(A.sub_count, 1);
+            float v = 0.0f;
+            if (lane < (patch ? 25 : 1)) v = tc2_exact(o.D[lane], o.s1[lane], o.s2[lane], mean, nn, cnorm, A.measure);
+            if (patch) {
+                slot = __shfl_sync(kFull, slot, 0);
+                if (lane < 25) A.sub_patch[static_cast<int64_t>(slot) * 25 + lane] = v;
+                if (lane == 0) {
+                    A.sub_point[slot] = o.k;
+                    A.sub_origin[2 * slot] = o.pi;
+                    A.sub_origin[2 * slot + 1] = o.pj;
+                }
+            } else if (lane == 0) {
+                A.out.dx[o.k] = __double2float_rn(__dadd_rn(static_cast<double>(o.pj - o.nc / 2), A.pts.dx0[o.k]));
+                A.out.dy[o.k] = __double2float_rn(__dadd_rn(static_cast<double>(o.pi - o.nr / 2), A.pts.dy0[o.k]));
+                A.out.corr[o.k] = v;
+            }
+            __syncwarp();
+        }
+    } else {
+    // ------------------------------------------------------------------------------------ main
+    uint32_t phase = 0, ph = 0;
+    bool failed = false;
+    int mb = 0;  // the slot of the next measured point's result
+    clear_acc();
+    int dirty_ch = 0;
+    // This thread's row of the chip operand and its first chip column (the same for every point).
+    const int e_groups = kTcThreads / A.NB;  // 0: more rows than threads
+    const int e_row = tid % A.NB, e_grp = tid / A.NB;
+    TC_PHASE_INIT
+    // Whether s_S1, s_S2 and s_R hold the previous point's box sums, as rings of NRS rows per
+    // column: surface row i of that point is at row (i + rbase) mod NRS, so carrying the sums
+    // down by `sh` rows advances rbase instead of moving them. s_L1, s_L2: its column sums of the
+    // last surface row.
     bool held = false;
-    int64_t h_wr = 0, h_wc = 0;
-    // s_S1 / s_S2 are rings of NRS rows per column: surface row i of the held point is stored at
-    // row (i + rbase) mod NRS, so carrying the sums down by `sh` rows advances rbase instead of
-    // moving them.
     int rbase = 0;
     auto ring = [&](int i) {
         const int r = i + rbase;
         return r >= A.NRS ? r - A.NRS : r;
     };
-    int h_ch = 0, h_cw = 0, h_nr = 0, h_nc = 0;
-    for (int64_t k = kbeg; k < kend; ++k, ++iter) {
-        tc::cp_async_wait_all();  // no copy of a skipped point is still landing
-        tc::fence_before_sync();
-        __syncthreads();  // the previous point's buffers and accumulators are no longer read
-        tc::fence_after_sync();
+    for (int b = 0;; b ^= 1, ph ^= 1u) {
+        // A wait that runs out leaves this thread with an empty point until the next barrier, where
+        // all of them leave.
+        const bool got = tc::mbar_wait(&s_full, ph, kTcWaitPolls);
+        if (!got) s_fail = 1;
         TC_PHASE(0)
-        const int ib = iter & 1;
-        if (tid < 2) s_isum[ib ^ 1][tid] = 0ull;
-        // The geometry: computed ahead by the previous iteration when it reached its products.
-        PtGeo g;
-        if (s_geo[ib].k == k) {
-            g = s_geo[ib];
-        } else {
-            pt_geometry(A, k, g);
+        const Tc2Pt& g = s_pt[b];
+        const int64_t k = got ? g.k : 0;
+        if (k < 0) {
+            bar_main_or(false);
+            break;
         }
-        if (!g.ok) continue;
-        const int ch = g.ch, cw = g.cw, nr = g.nr, nc = g.nc, prx = g.prx, pry = g.pry;
-        TC_PHASE(1)
+        const int ch = got ? g.ch : 0, cw = got ? g.cw : 0, nr = got ? g.nr : 0, nc = got ? g.nc : 0;
         const int64_t chip_r = g.chip_r, chip_c = g.chip_c, win_r = g.win_r, win_c = g.win_c;
-        const long long nnl = static_cast<long long>(ch) * cw;
-        const bool pow2 = (nnl & (nnl - 1)) == 0 && nnl <= 4096;
-
-        // The window's columns as aligned 16-byte chunks, copied asynchronously (cp.async) into
-        // the column-sum buffer -- free until the box sums -- while the chip is staged: when
-        // every row of the window lies in the image, a column takes the Q + 1 chunks from the
-        // aligned address at or below its first row (columns whose chunks would leave the array,
-        // and windows that reach outside the image's rows, are staged from global memory below).
-        const int Q = (ch + nr - 1 + 15) / 16;
-        const int RQ = Q + 1;
-        uint8_t* s_Wraw = reinterpret_cast<uint8_t*>(s_V1);
-        const bool rows_in = win_r >= 0 && win_r + 16 * Q <= A.nrows;
-        auto raw_col = [&](int x, const uint8_t** first) {
-            // Column x's aligned first chunk when all its chunks are inside the array, else null.
-            const int64_t c = win_c + x;
-            if (!rows_in || c < 0 || c >= A.ncols) return false;
-            const uint8_t* p = A.ref + c * A.nrows + win_r;
-            const uint8_t* a0 = reinterpret_cast<const uint8_t*>(reinterpret_cast<uintptr_t>(p) & ~uintptr_t(15));
-            if (a0 < A.ref || a0 + 16 * RQ > ref_end) return false;
-            *first = a0;
-            return true;
-        };
-        if (rows_in) {
-            for (int it = tid; it < A.XS * RQ; it += bd) {
-                const int x = it / RQ, kq = it - x * RQ;
-                const uint8_t* a0;
-                if (raw_col(x, &a0)) tc::cp_async16(s_Wraw + static_cast<size_t>(it) * 16, a0 + 16 * kq);
-            }
+        const int raw = g.raw;
+        const int nnl = ch * cw;
+        const bool pow2 = tc2_exact_sums(nnl);
+        const int Q = (ch + nr - 1 + 15) / 16, XW = cw + nc - 1;
+        Tc2Out& out = s_out[mb];
+        // Carried box sums: the previous point (its slot is still in place) has the same window
+        // columns and shape `sh` rows higher; only surface rows iA .. nr - 1 are new.
+        int iA = 0;
+        {
+            const Tc2Pt& h = s_pt[b ^ 1];
+            const int64_t sh = win_r - h.win_r;
+            if (held && win_c == h.win_c && ch == h.ch && cw == h.cw && nr == h.nr && nc == h.nc &&
+                sh > 0 && sh < nr)
+                iA = nr - static_cast<int>(sh);
+            held = false;
         }
-        tc::cp_async_commit();
 
-        // The chip as zero-padded byte columns, _any_valid over it (src/track.jl:416-421) and,
-        // for power-of-two areas, its exact integer sums (as in k_corr_tc).
+        // The chip as zero-padded byte columns, _any_valid over it (src/track.jl:416-421) and its
+        // exact integer sums; the window as blocks W[16 q + r][x] of 16 rows. A task is 16 rows of
+        // one column, from the two chunks that hold them (or from global memory at the image's
+        // border) shifted into place.
         int any = 0;
-        unsigned long long isum = 0ull, isq = 0ull;
+        uint32_t isum = 0u, isq = 0u;
         if (ch < dirty_ch)
-            for (int b = warp; b < A.CWM; b += nwarps)
-                for (int a = ch + lane; a < dirty_ch; a += 32) s_P[b * A.PC + kPadL + a] = 0;
+            for (int c = warp; c < A.CWM; c += 8)
+                for (int a = ch + lane; a < dirty_ch; a += 32) s_P[c * A.PC + kPadL + a] = 0;
         dirty_ch = ch;
-        for (int a0 = 0; a0 < ch; a0 += 32) {
-            const int a = a0 + lane;
-            const int64_t r = chip_r + a;
-            const bool rin = a < ch && r >= 0 && r < A.nrows;
-            constexpr int kU = 4;
-            for (int b0 = warp; b0 < cw; b0 += kU * nwarps) {
-                uint32_t v[kU], m[kU];
-#pragma unroll
-                for (int u = 0; u < kU; ++u) {
-                    const int b = b0 + u * nwarps;
-                    const int64_t c = chip_c + b;
-                    const bool in = rin && b < cw && c >= 0 && c < A.ncols;
-                    v[u] = in ? A.sec[r + c * A.nrows] : 0u;
-                    m[u] = in ? A.valid[r + c * A.nrows] : 0u;
-                }
-#pragma unroll
-                for (int u = 0; u < kU; ++u) {
-                    const int b = b0 + u * nwarps;
-                    if (a < ch && b < cw) {
-                        s_P[b * A.PC + kPadL + a] = static_cast<uint8_t>(v[u]);
-                        any |= m[u];
-                        isum += v[u];
-                        isq += v[u] * v[u];
+        {
+            const int nb16 = (ch + 15) >> 4, nct = nb16 * cw;
+            const uint32_t ld = static_cast<uint32_t>(A.nrows);
+            const uint32_t co = static_cast<uint32_t>(chip_c) * ld + static_cast<uint32_t>(chip_r);
+            const uint32_t cbase = tc2_low(A.sec) + co, mbase = tc2_low(A.valid) + co;
+            const uint32_t wbase = tc2_low(A.ref) + static_cast<uint32_t>(win_c) * ld + static_cast<uint32_t>(win_r);
+            // Window tasks: a column and half of its blocks (the chunk between two blocks is read
+            // once); chip tasks from the block's other end.
+            const int qh = (Q + 1) >> 1;
+            for (int w = tid; w < 2 * XW; w += kTcThreads) {
+                const int up = w >= XW ? 1 : 0, x = w - up * XW;
+                const int q0 = up * qh, q1 = min(q0 + qh, Q);
+                uint8_t* dst = s_W + q0 * A.QS + x * 16;
+                if (raw & 1) {
+                    Col16 L;
+                    L.s = (wbase + static_cast<uint32_t>(x) * ld) & 15u;
+                    const uint4* src = s_rawW + q0 * XW + x;
+                    L.lo = src[0];
+                    for (int q = q0; q < q1; ++q) {
+                        src += XW;
+                        L.hi = src[0];
+                        *reinterpret_cast<uint4*>(dst) = col16_finish(L);
+                        L.lo = L.hi;
+                        dst += A.QS;
+                    }
+                } else {
+                    for (int q = q0; q < q1; ++q) {
+                        *reinterpret_cast<uint4*>(dst) =
+                            tc2_border(A.ref, ref_end, A.nrows, A.ncols, win_c + x, win_r + 16 * q);
+                        dst += A.QS;
                     }
                 }
             }
-        }
-        if (pow2) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                isum += __shfl_xor_sync(kFull, isum, o);
-                isq += __shfl_xor_sync(kFull, isq, o);
-            }
-            if (lane == 0) {
-                atomicAdd(&s_isum[ib][0], isum);
-                atomicAdd(&s_isum[ib][1], isq);
-            }
-        }
-        tc::cp_async_wait_all();  // this thread's window chunks have landed (visible after the barrier)
-        if (!__syncthreads_or(any)) continue;
-        TC_PHASE(2)
-        if (tid == 0) A.out.searched[k] = 1;
-
-        double mean, sq, csum_d;
-        if (pow2) {
-            const long long cs = static_cast<long long>(s_isum[ib][0]);
-            const long long c2 = static_cast<long long>(s_isum[ib][1]);
-            csum_d = static_cast<double>(cs);
-            mean = __ddiv_rn(csum_d, static_cast<double>(nnl));
-            sq = __ddiv_rn(static_cast<double>(nnl * c2 - cs * cs), static_cast<double>(nnl));
-        } else {
-            staged_chip_stats(s_P, A.PC, ch, cw, tid, bd, s_red, &csum_d, &mean, &sq);
-        }
-        if (!(sq > __dmul_rn(__dmul_rn(DBL_EPSILON, static_cast<double>(ch)), static_cast<double>(cw))))
-            continue;  // degenerate chip: searched, no measurement (src/track.jl:286)
-        TC_PHASE(3)
-        const double cnorm = __dsqrt_rn(sq);
-        if (tid == 0 && !(A.up == 1 || nr < 5 || nc < 5)) s_slot = atomicAdd(A.sub_count, 1);
-        const double nn = static_cast<double>(nnl);
-
-        // Window blocks W[16 q + r][x] (x < XS) from the window's first row: from the chunks in
-        // shared memory, or from global memory for the columns that have none.
-        const int XW = cw + nc - 1;
-        for (int q = warp; q < Q; q += nwarps)
-            for (int x = lane; x < A.XS; x += 32) {
-                const uint8_t* a0;
-                Col16 L;
-                if (raw_col(x, &a0)) {
-                    const uint4* rc = reinterpret_cast<const uint4*>(s_Wraw + static_cast<size_t>(x * RQ + q) * 16);
+            for (int t = kTcThreads - 1 - tid; t < nct; t += kTcThreads) {
+                const int kb = t / cw, c = t - kb * cw;
+                uint4 v, mk;
+                if (raw & 2) {
+                    const uint4* rc = s_rawC + kb * cw + c;
+                    const uint4* rm = rc + (nb16 + 1) * cw;
+                    Col16 L;
                     L.lo = rc[0];
-                    L.hi = rc[1];
-                    L.s = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(A.ref + (win_c + x) * A.nrows + win_r) & 15);
+                    L.hi = rc[cw];
+                    L.s = (cbase + static_cast<uint32_t>(c) * ld) & 15u;
+                    v = col16_finish(L);
+                    L.lo = rm[0];
+                    L.hi = rm[cw];
+                    L.s = (mbase + static_cast<uint32_t>(c) * ld) & 15u;
+                    mk = col16_finish(L);
                 } else {
-                    L = col16_issue(A.ref, ref_end, A.nrows, A.ncols, win_c + x, win_r + 16 * q);
+                    v = tc2_border(A.sec, sec_end, A.nrows, A.ncols, chip_c + c, chip_r + 16 * kb);
+                    mk = tc2_border(A.valid, valid_end, A.nrows, A.ncols, chip_c + c, chip_r + 16 * kb);
                 }
-                *reinterpret_cast<uint4*>(s_W + q * A.QS + x * 16) = col16_finish(L);
+                const int keep = ch - 16 * kb;
+                uint32_t w[4] = {v.x, v.y, v.z, v.w}, mw[4] = {mk.x, mk.y, mk.z, mk.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int n = keep - 4 * i;
+                    const uint32_t m = n >= 4 ? 0xffffffffu : n <= 0 ? 0u : (1u << (8 * n)) - 1u;
+                    w[i] &= m;
+                    any |= (mw[i] & m) != 0u;
+                    isum = __dp4a(w[i], 0x01010101u, isum);
+                    isq = __dp4a(w[i], w[i], isq);
+                }
+                *reinterpret_cast<uint4*>(s_P + c * A.PC + kPadL + 16 * kb) =
+                    make_uint4(w[0], w[1], w[2], w[3]);
             }
-        // E: NB rows per chip column, row e (u = e - NB + 16) = 16 bytes from chip row -u.
-        {
-            const int nrow = cw * A.NB;
-            int bl = tid / A.NB, e = tid - bl * A.NB;
-            const int sbl = bd / A.NB, se = bd - sbl * A.NB;
-            for (int t = tid; t < nrow; t += bd) {
-                const int src = bl * A.PC + kPadL - 16 + A.NB - e;
-                const uint32_t* w = reinterpret_cast<const uint32_t*>(s_P + (src & ~3));
-                const uint32_t sh = static_cast<uint32_t>(src & 3) * 8u;
-                uint4 o;
-                o.x = __funnelshift_r(w[0], w[1], sh);
-                o.y = __funnelshift_r(w[1], w[2], sh);
-                o.z = __funnelshift_r(w[2], w[3], sh);
-                o.w = __funnelshift_r(w[3], w[4], sh);
-                *reinterpret_cast<uint4*>(s_E + bl * A.PS + e * 16) = o;
-                bl += sbl;
-                e += se;
-                if (e >= A.NB) {
-                    e -= A.NB;
-                    ++bl;
+        }
+        if (pow2) {  // at most 4096 pixels: sums below 2^20 and 2^28
+            isum = __reduce_add_sync(kFull, isum);
+            isq = __reduce_add_sync(kFull, isq);
+            if (lane == 0 && isq != 0u) {
+                atomicAdd(&s_isum[b][0], isum);
+                atomicAdd(&s_isum[b][1], isq);
+            }
+        }
+        const bool seen = bar_main_or(any);
+        if (s_fail) {
+            failed = true;
+            break;
+        }
+        TC_PHASE(1)
+        const uint32_t cs = s_isum[b][0], c2 = s_isum[b][1];
+        if (tid == 0) {
+            if (seen) A.out.searched[k] = 1;
+            s_isum[b ^ 1][0] = s_isum[b ^ 1][1] = 0u;  // for the next point
+        }
+        // prepare_chip! statistics. Power-of-two areas: the sum of squared deviations is
+        // (nn sum(C^2) - sum(C)^2) / nn exactly, degenerate only when that integer is 0 (1 / nn is
+        // above the threshold); the helper makes mean and norm. Other areas: the CUDA-core
+        // kernel's FP64 sums.
+        const unsigned long long nsq =
+            static_cast<unsigned long long>(nnl) * c2 - static_cast<unsigned long long>(cs) * cs;
+        bool measured = seen;
+        if (seen) {
+            if (pow2) {
+                measured = nsq != 0ull;
+            } else {
+                double mean, sq, csum_d;
+                staged_chip_stats<true>(s_P, A.PC, ch, cw, tid, kTcThreads, s_red, &csum_d, &mean, &sq);
+                measured = sq > __dmul_rn(__dmul_rn(DBL_EPSILON, static_cast<double>(ch)), static_cast<double>(cw));
+                if (measured && tid == 0) {
+                    out.mean = mean;
+                    out.sq = sq;
+                    out.csum = csum_d;
                 }
             }
         }
-        // The products add into accumulator columns [0, round16(nr)): surface row i is column i.
-        const int dcols = (nr + 15) & ~15;
-        if (warp < 4) {
-            // Clear the columns the products add into (one lane quarter per warp).
-            uint32_t z[16];
-#pragma unroll
-            for (int t = 0; t < 16; ++t) z[t] = 0u;
-            const uint32_t lq = taddr + (static_cast<uint32_t>(32 * warp) << 16);
-            for (int c = 0; c < dcols; c += 16)
-#pragma unroll
-                for (int t = 0; t < kTc2Issuers; ++t)
-                    tc::tmem_st16(lq + static_cast<uint32_t>(t) * acc1 + static_cast<uint32_t>(c), z);
-            tc::tmem_wait_st();
+        if (!measured) {  // not searched, or degenerate: no measurement (src/track.jl:286)
+            bar_main();
+            if (tid == 0) tc::mbar_arrive(&s_free);
+            continue;
         }
+        TC_PHASE(2)
+
+        // E: NB rows per chip column, row e (u = e - NB + 16) = 16 bytes from chip row -u. A thread
+        // keeps its row, so its byte shift is fixed.
+        auto build_row = [&](int e, int c) {
+            const int src = c * A.PC + kPadL - 16 + A.NB - e;
+            const uint32_t* w = reinterpret_cast<const uint32_t*>(s_P + (src & ~3));
+            const uint32_t sh = static_cast<uint32_t>(src & 3) * 8u;
+            uint4 o;
+            o.x = __funnelshift_r(w[0], w[1], sh);
+            o.y = __funnelshift_r(w[1], w[2], sh);
+            o.z = __funnelshift_r(w[2], w[3], sh);
+            o.w = __funnelshift_r(w[3], w[4], sh);
+            *reinterpret_cast<uint4*>(s_E + c * A.PS + e * 16) = o;
+        };
+        if (e_grp < e_groups)
+            for (int c = e_grp; c < cw; c += e_groups) build_row(e_row, c);
+        if (tid == 0) {
+            out.k = k;
+            out.nr = nr;
+            out.nc = nc;
+            out.nn = nnl;
+            out.cs = cs;
+            out.c2 = c2;
+            s_more[mb] = 1;
+        }
+        // The products add into accumulator columns [0, round16(nr)): surface row i is column i. The
+        // accumulators were cleared when the previous point's were read.
+        tc::tmem_wait_st();
         tc::fence_proxy_async_smem();
         tc::fence_before_sync();
-        __syncthreads();  // s_P, s_W, s_E complete; accumulator cleared
-        TC_PHASE(4)
-        // Lane 0 of the last kTc2Issuers warps issue the products, each for a share of the chip
-        // column pairs into its own accumulator (one thread issues an MMA about every 120
-        // cycles; several issuers interleave theirs).
-        if (lane == 0 && warp >= nwarps - kTc2Issuers) {
-            const int stream = nwarps - 1 - warp;
-            tc::fence_after_sync();
-#ifdef AR_TC_PHASES
-            const unsigned long long tmi0 = clock64();
-#endif
-            // Descriptors advance by adding to their start-address field, the low bits of the
-            // low word (16-byte units; shared addresses stay below 2^18, so nothing carries):
-            // a product costs the issuing thread two 32-bit adds and the MMA itself.
-            const uint64_t da0 = tc::smem_desc(tc::smem_u32(s_W), 16, 128);
-            const uint64_t db0 = tc::smem_desc(tc::smem_u32(s_E), A.PS, 128);
-            const uint32_t a_hi = static_cast<uint32_t>(da0 >> 32);
-            const uint32_t b_hi = static_cast<uint32_t>(db0 >> 32);
-            const uint32_t bstep = static_cast<uint32_t>(2 * A.PS) >> 4;
-            const int pairs = cw / 2;
-            const int t_begin = pairs * stream / kTc2Issuers;
-            const int npairs = pairs * (stream + 1) / kTc2Issuers - t_begin;
-            for (int q = 0; q < Q; ++q) {
-                // Only the operand rows e in [elo, elo + n) of block q reach surface rows.
-                int elo, n;
-                if (!block_rows(q, A.NB, nr, &elo, &n)) continue;
-                const uint32_t idesc = tc::idesc_u8_s32(64, n);
-                uint32_t a_lo = static_cast<uint32_t>(da0) +
-                                static_cast<uint32_t>(q * A.QS >> 4) + 2u * static_cast<uint32_t>(t_begin);
-                uint32_t b_lo = static_cast<uint32_t>(db0) + static_cast<uint32_t>(elo) +
-                                bstep * static_cast<uint32_t>(t_begin);
-                const uint32_t dn = taddr + static_cast<uint32_t>(stream) * acc1 +
-                                    static_cast<uint32_t>(16 * q + elo - (A.NB - 16));
-                int t = 0;
-                for (; t + 4 <= npairs; t += 4) {
-                    tc::mma_u8_halves(dn, a_lo, a_hi, b_lo, b_hi, idesc);
-                    tc::mma_u8_halves(dn, a_lo + 2, a_hi, b_lo + bstep, b_hi, idesc);
-                    tc::mma_u8_halves(dn, a_lo + 4, a_hi, b_lo + 2 * bstep, b_hi, idesc);
-                    tc::mma_u8_halves(dn, a_lo + 6, a_hi, b_lo + 3 * bstep, b_hi, idesc);
-                    a_lo += 8;
-                    b_lo += 4 * bstep;
-                }
-                for (; t < npairs; ++t) {
-                    tc::mma_u8_halves(dn, a_lo, a_hi, b_lo, b_hi, idesc);
-                    a_lo += 2;
-                    b_lo += bstep;
-                }
+        bar_products();  // s_P, s_W, s_E complete; accumulators clear; the chunks are read
+        TC_PHASE(3)
+        // The reciprocal root of a value's variance term (below).
+        const float nnf = static_cast<float>(nnl);
+        auto recip = [&](float s1, uint32_t s2u) {
+            const float s2 = __uint2float_rn(s2u);
+            float vx = s2;
+            if (A.measure != AR_NCC) {
+                const float q = __fmul_rn(s1, s1);
+                vx = __fmaf_rn(nnf, s2, -q);
+                if (__fmaf_rn(nnf, s2, q) > 2048.0f * vx) vx = -1.0f;  // its root is NaN
             }
-            tc::mma_commit(&s_mbar);
-#ifdef AR_TC_PHASES
-            // Profiling builds: time to issue the products, then until they complete.
-            const unsigned long long tmi1 = clock64();
-            if (stream == 0) {
-                tc::mbar_wait(&s_mbar, phase, kTcWaitPolls);
-                tmi_issue += tmi1 - tmi0;
-                tmi_done += clock64() - tmi1;
-            }
-#endif
-            // The next point's geometry, read after the next loop-top barrier.
-            const int64_t kn = k + 1;
-            if (stream == 0 && kn < kend) pt_geometry(A, kn, s_geo[ib ^ 1]);
-        }
-        TC_PHASE(5)
-        // S[j][i] = sums of V[i][j .. j + cw - 1] for rows i in [i_lo, i_lo + ni): a task is a
-        // row i and 16 columns j (the warps that do not issue products).
-        auto box_rows = [&](int i_lo, int ni) {
-            constexpr int kBT = kTcThreads - 32 * kTc2Issuers;
-            const int jseg = (nc + 15) >> 4;
-            const bool vec = (cw & 3) == 0;
-            for (int task = tid; task < ni * jseg; task += kBT) {
-                const int sg = task / ni, i = i_lo + (task - sg * ni);
-                const int j0 = 16 * sg;
-                const uint32_t* r1 = s_V1 + i * A.XV;
-                const uint32_t* r2 = s_V2 + i * A.XV;
-                uint32_t g1 = 0, g2 = 0;
-                int bb = 0;
-                for (; bb + 4 <= cw; bb += 4) {
-                    const uint4 v = *reinterpret_cast<const uint4*>(r1 + j0 + bb);
-                    const uint4 w = *reinterpret_cast<const uint4*>(r2 + j0 + bb);
-                    g1 += (v.x + v.y) + (v.z + v.w);
-                    g2 += (w.x + w.y) + (w.z + w.w);
-                }
-                for (; bb < cw; ++bb) {
-                    g1 += r1[j0 + bb];
-                    g2 += r2[j0 + bb];
-                }
-#pragma unroll
-                for (int u4 = 0; u4 < 16; u4 += 4) {
-                    const uint4 o1 = *reinterpret_cast<const uint4*>(r1 + j0 + u4);
-                    const uint4 o2 = *reinterpret_cast<const uint4*>(r2 + j0 + u4);
-                    uint4 i1, i2;
-                    if (vec) {
-                        i1 = *reinterpret_cast<const uint4*>(r1 + j0 + u4 + cw);
-                        i2 = *reinterpret_cast<const uint4*>(r2 + j0 + u4 + cw);
-                    } else {
-                        const uint32_t* p1 = r1 + j0 + u4 + cw;
-                        const uint32_t* p2 = r2 + j0 + u4 + cw;
-                        i1 = make_uint4(p1[0], p1[1], p1[2], p1[3]);
-                        i2 = make_uint4(p2[0], p2[1], p2[2], p2[3]);
-                    }
-                    const uint32_t oo1[4] = {o1.x, o1.y, o1.z, o1.w}, ii1[4] = {i1.x, i1.y, i1.z, i1.w};
-                    const uint32_t oo2[4] = {o2.x, o2.y, o2.z, o2.w}, ii2[4] = {i2.x, i2.y, i2.z, i2.w};
-#pragma unroll
-                    for (int m = 0; m < 4; ++m) {
-                        const int j = j0 + u4 + m;
-                        if (j < nc) {
-                            s_S1[j * A.NRS + i] = g1;
-                            s_S2[j * A.NRS + i] = g2;
-                            g1 = g1 + ii1[m] - oo1[m];
-                            g2 = g2 + ii2[m] - oo2[m];
-                        }
-                    }
-                }
-            }
+            return s2u == 0u ? 0.0f : rsqrtf(vx);
         };
-        // Box sums of W and W^2 (integral_both!, boxsum, src/integral.jl:141-170, 244-247) as
-        // exact integers, warps 0-4 (named barrier 1) while warps 5-7 issue the products. When
-        // the held sums belong to the same window geometry `sh` rows higher, the ring's base
-        // advances by `sh` (the held rows become rows 0 .. nr - sh - 1) and only the last `sh`
-        // rows are computed.
-        const int64_t sh64 = win_r - h_wr;
-        const bool carry = held && win_c == h_wc && ch == h_ch && cw == h_cw && nr == h_nr &&
-                           nc == h_nc && sh64 > 0 && sh64 < nr;
+        const bool carry = iA > 0;
         if (carry) {
-            rbase += static_cast<int>(sh64);
+            rbase += nr - iA;
             if (rbase >= A.NRS) rbase -= A.NRS;
         } else {
             rbase = 0;
@@ -2288,336 +2449,489 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_corr_tc2(const TcArgs A) {
 #ifdef AR_TC_PHASES
         if (tid == 0 && carry) atomicAdd(&g_tc_phase[14], 1ull);
 #endif
-        if (warp < nwarps - kTc2Issuers) {
-            constexpr int kBT = kTcThreads - 32 * kTc2Issuers;
-            if (carry) {
-                const int sh = static_cast<int>(sh64);
-                // Column sums of the new rows i in [nr - sh, nr): an item is a window column and
-                // up to 4 consecutive rows; its first sum from 4-byte groups (dp4a), then a
-                // sliding update. The row groups of a column are adjacent lanes: their words lie
-                // in different banks of the column's 16-byte block.
-                const int i0 = nr - sh;
-                const int nparts = (sh + 3) >> 2;
-                for (int item = tid; item < XW * nparts; item += kBT) {
-                    const int x = item / nparts, pt = item - x * nparts;
-                    const int ia = i0 + 4 * pt, ie = min(ia + 4, nr);
-                    const uint8_t* colx = s_W + x * 16;
-                    // Rows r .. r + 3 of column x as one word (a group may cross a block).
-                    auto word = [&](int r) {
-                        const int rb = r >> 4, o = r & 15, ow = o & ~3;
-                        const uint32_t lo = *reinterpret_cast<const uint32_t*>(colx + rb * A.QS + ow);
-                        if ((o & 3) == 0) return lo;
-                        const int nb = ow + 4 < 16 ? rb : rb + 1, no = ow + 4 < 16 ? ow + 4 : 0;
-                        const uint32_t hi = nb < Q ? *reinterpret_cast<const uint32_t*>(colx + nb * A.QS + no) : 0u;
-                        return __funnelshift_r(lo, hi, 8u * static_cast<uint32_t>(o & 3));
-                    };
-                    uint32_t h1 = 0, h2 = 0;
-                    int a = 0;
-                    for (; a + 4 <= ch; a += 4) {
-                        const uint32_t w = word(ia + a);
-                        h1 = __dp4a(w, 0x01010101u, h1);
-                        h2 = __dp4a(w, w, h2);
-                    }
-                    if (a < ch) {
-                        const uint32_t mk = (1u << (8 * (ch - a))) - 1u;
-                        const uint32_t w = word(ia + a) & mk;
-                        h1 = __dp4a(w, 0x01010101u, h1);
-                        h2 = __dp4a(w, w, h2);
-                    }
-                    for (int i = ia; i < ie; ++i) {
-                        s_V1[i * A.XV + x] = h1;
-                        s_V2[i * A.XV + x] = h2;
-                        if (i + 1 < ie) {
-                            const uint32_t o = colx[(i >> 4) * A.QS + (i & 15)];
-                            const int R = i + ch;
-                            const uint32_t n = colx[(R >> 4) * A.QS + (R & 15)];
-                            h1 = h1 + n - o;
-                            h2 = h2 + n * n - o * o;
-                        }
+        const int nbox = kTcThreads - 32 * A.issuers;  // the threads that sum the boxes
+        if (tid >= nbox) {
+            // Each issuing thread takes a share of the chip column pairs (one thread issues an MMA
+            // about every 120 cycles; several issuers, and other CTAs, interleave theirs).
+            if (lane == 0) {
+                const int stream = 7 - warp;
+                tc::fence_after_sync();
+#ifdef AR_TC_PHASES
+                const unsigned long long tmi0 = clock64();
+#endif
+                // Descriptors advance by adding to their start-address field, the low bits of the
+                // low word (16-byte units; shared addresses stay below 2^18, so nothing carries):
+                // a product costs the issuing thread two 32-bit adds and the MMA itself.
+                const uint64_t da0 = tc::smem_desc(tc::smem_u32(s_W), 16, 128);
+                const uint64_t db0 = tc::smem_desc(tc::smem_u32(s_E), A.PS, 128);
+                const uint32_t a_hi = static_cast<uint32_t>(da0 >> 32);
+                const uint32_t b_hi = static_cast<uint32_t>(db0 >> 32);
+                const uint32_t bstep = static_cast<uint32_t>(2 * A.PS) >> 4;
+                const int pairs = cw / 2;
+                const int t_begin = pairs * stream / A.issuers;
+                const int npairs = pairs * (stream + 1) / A.issuers - t_begin;
+                for (int q = 0; q < Q; ++q) {
+                    // Only the operand rows e in [elo, elo + n) of block q reach surface rows.
+                    int elo, n;
+                    if (!block_rows(q, A.NB, nr, &elo, &n)) continue;
+                    const uint32_t idesc = tc::idesc_u8_s32(64, n);
+                    uint32_t a_lo = static_cast<uint32_t>(da0) +
+                                    static_cast<uint32_t>(q * A.QS >> 4) + 2u * static_cast<uint32_t>(t_begin);
+                    uint32_t b_lo = static_cast<uint32_t>(db0) + static_cast<uint32_t>(elo) +
+                                    bstep * static_cast<uint32_t>(t_begin);
+                    const uint32_t dn = taddr + static_cast<uint32_t>(stream) * acc1 +
+                                        static_cast<uint32_t>(16 * q + elo - (A.NB - 16));
+                    for (int t = 0; t < npairs; ++t) {
+                        tc::mma_u8_halves(dn, a_lo, a_hi, b_lo, b_hi, idesc);
+                        a_lo += 2;
+                        b_lo += bstep;
                     }
                 }
-                asm volatile("bar.sync 1, %0;" ::"r"(kBT) : "memory");
-                // Row sums of the new rows: a task is a row and 4 consecutive columns j.
-                const int ng = (nc + 3) >> 2;
-                for (int task = tid; task < sh * ng; task += kBT) {
-                    const int g = task / sh, i = i0 + (task - g * sh);
-                    const int j0 = 4 * g;
-                    const uint32_t* r1 = s_V1 + i * A.XV;
-                    const uint32_t* r2 = s_V2 + i * A.XV;
-                    uint32_t g1 = 0, g2 = 0;
-                    int bb = 0;
-                    for (; bb + 4 <= cw; bb += 4) {
-                        const uint4 v = *reinterpret_cast<const uint4*>(r1 + j0 + bb);
-                        const uint4 w = *reinterpret_cast<const uint4*>(r2 + j0 + bb);
-                        g1 += (v.x + v.y) + (v.z + v.w);
-                        g2 += (w.x + w.y) + (w.z + w.w);
-                    }
-                    for (; bb < cw; ++bb) {
-                        g1 += r1[j0 + bb];
-                        g2 += r2[j0 + bb];
-                    }
-                    // Outgoing and incoming columns as 16-byte loads (rows stay inside XV).
-                    const uint4 o1 = *reinterpret_cast<const uint4*>(r1 + j0);
-                    const uint4 o2 = *reinterpret_cast<const uint4*>(r2 + j0);
-                    uint4 i1, i2;
-                    if ((cw & 3) == 0) {
-                        i1 = *reinterpret_cast<const uint4*>(r1 + j0 + cw);
-                        i2 = *reinterpret_cast<const uint4*>(r2 + j0 + cw);
-                    } else {
-                        const uint32_t* p1 = r1 + j0 + cw;
-                        const uint32_t* p2 = r2 + j0 + cw;
-                        i1 = make_uint4(p1[0], p1[1], p1[2], p1[3]);
-                        i2 = make_uint4(p2[0], p2[1], p2[2], p2[3]);
-                    }
-                    const uint32_t oo1[4] = {o1.x, o1.y, o1.z, o1.w}, ii1[4] = {i1.x, i1.y, i1.z, i1.w};
-                    const uint32_t oo2[4] = {o2.x, o2.y, o2.z, o2.w}, ii2[4] = {i2.x, i2.y, i2.z, i2.w};
-                    const int ri = ring(i);
+                tc::mma_commit(&s_mbar);
+#ifdef AR_TC_PHASES
+                if (stream == 0) atomicAdd(&g_tc_phase[12], clock64() - tmi0);
+#endif
+            }
+            __syncwarp();
+        } else {
+            // Box sums of W and W^2 (integral_both!, boxsum, src/integral.jl:141-170, 244-247) as
+            // exact integers, beside the products: column sums V of ch rows, then sums of cw
+            // columns of V, s1 kept as Float32 (exact: below 2^24) and s2. VR surface rows at a
+            // time.
+            const int kBT = nbox;
+            auto bar_box = [&]() { asm volatile("bar.sync 1, %0;" ::"r"(kBT) : "memory"); };
+            if (carry) {
+                // The held sums belong to the same window geometry `sh` rows higher: only the last
+                // `sh` rows are new. Their column sums slide on from the held last row (s_L).
+                for (int i0 = iA; i0 < nr; i0 += A.VR) {
+                    const int ni = min(A.VR, nr - i0);
+                    for (int x = tid; x < XW; x += kBT) {
+                        const uint8_t* colx = s_W + x * 16;
+                        auto word = [&](int a) {  // rows a .. a + 3, a a multiple of 4
+                            const int q = min(a >> 4, Q - 1);
+                            return *reinterpret_cast<const uint32_t*>(colx + q * A.QS + (a & 12));
+                        };
+                        // Row i's sum drops window row i - 1 and takes row i - 1 + ch.
+                        const int R0 = i0 - 1, R1 = i0 - 1 + ch;
+                        const uint32_t so = static_cast<uint32_t>(R0 & 3) * 8u;
+                        const uint32_t sn = static_cast<uint32_t>(R1 & 3) * 8u;
+                        int ao = R0 & ~3, an = R1 & ~3;
+                        uint32_t lo_o = word(ao), lo_n = word(an);
+                        uint32_t h1 = s_L1[x], h2 = s_L2[x];
+                        uint32_t* v1 = s_V1 + x;
+                        uint32_t* v2 = s_V2 + x;
+                        for (int i = 0; i < ni; i += 4) {
+                            ao += 4;
+                            an += 4;
+                            const uint32_t hi_o = word(ao), hi_n = word(an);
+                            const uint32_t wo = __funnelshift_r(lo_o, hi_o, so);
+                            const uint32_t wn = __funnelshift_r(lo_n, hi_n, sn);
+                            lo_o = hi_o;
+                            lo_n = hi_n;
 #pragma unroll
-                    for (int m = 0; m < 4; ++m) {
-                        const int j = j0 + m;
-                        if (j < nc) {
-                            s_S1[j * A.NRS + ri] = g1;
-                            s_S2[j * A.NRS + ri] = g2;
-                            g1 = g1 + ii1[m] - oo1[m];
-                            g2 = g2 + ii2[m] - oo2[m];
+                            for (int u = 0; u < 4; ++u) {
+                                if (i + u < ni) {
+                                    const uint32_t bo = (wo >> (8 * u)) & 255u, bn = (wn >> (8 * u)) & 255u;
+                                    h1 += bn - bo;
+                                    h2 += bn * bn - bo * bo;
+                                    *v1 = h1;
+                                    *v2 = h2;
+                                }
+                                v1 += A.XV;
+                                v2 += A.XV;
+                            }
+                        }
+                        s_L1[x] = h1;
+                        s_L2[x] = h2;
+                    }
+                    bar_box();
+                    // Sums of cw columns as differences of prefix sums (exact modulo 2^32), a warp
+                    // per row.
+                    for (int il = warp; il < ni; il += kBT >> 5) {
+                        uint32_t* v1 = s_V1 + il * A.XV;
+                        uint32_t* v2 = s_V2 + il * A.XV;
+                        uint32_t c1 = 0u, c2_ = 0u;
+                        for (int x0 = 0; x0 < XW; x0 += 128) {
+                            const int x = x0 + 4 * lane;
+                            uint4 a = make_uint4(0, 0, 0, 0), d = a;
+                            if (x < XW) {
+                                a = *reinterpret_cast<const uint4*>(v1 + x);
+                                d = *reinterpret_cast<const uint4*>(v2 + x);
+                            }
+                            a.y += a.x;
+                            a.z += a.y;
+                            a.w += a.z;
+                            d.y += d.x;
+                            d.z += d.y;
+                            d.w += d.z;
+                            const uint32_t t1 = warp_inclusive_scan(a.w), t2 = warp_inclusive_scan(d.w);
+                            const uint32_t p1 = t1 - a.w + c1, p2 = t2 - d.w + c2_;
+                            if (x < XW) {
+                                *reinterpret_cast<uint4*>(v1 + x) = make_uint4(a.x + p1, a.y + p1, a.z + p1, a.w + p1);
+                                *reinterpret_cast<uint4*>(v2 + x) = make_uint4(d.x + p2, d.y + p2, d.z + p2, d.w + p2);
+                            }
+                            c1 += __shfl_sync(kFull, t1, 31);
+                            c2_ += __shfl_sync(kFull, t2, 31);
+                        }
+                        __syncwarp();
+                        const int ri = ring(i0 + il);
+                        for (int j = lane; j < nc; j += 32) {
+                            const float s1 = __uint2float_rn(v1[j + cw - 1] - (j > 0 ? v1[j - 1] : 0u));
+                            const uint32_t s2 = v2[j + cw - 1] - (j > 0 ? v2[j - 1] : 0u);
+                            const int o = j * A.NRS + ri;
+                            s_S1[o] = s1;
+                            s_S2[o] = s2;
+                            s_R[o] = recip(s1, s2);
                         }
                     }
+                    if (i0 + ni < nr) bar_box();
                 }
             } else {
                 // V[i][x] = sums over rows i .. i + ch - 1 of column x: a task is a column and the 16
                 // rows i of one block; its outgoing rows are that block, its incoming rows start ch
                 // rows lower.
-                const int nseg = (nr + 15) >> 4;
                 const int chb = ch >> 4, chr = ch & 15;
-                for (int task = tid; task < XW * nseg; task += kBT) {
-                    const int sgi = task / XW, x = task - sgi * XW;
-                    const int i0 = 16 * sgi;
-                    const uint8_t* colx = s_W + x * 16;
-                    const uint4 bo = *reinterpret_cast<const uint4*>(colx + sgi * A.QS);
-                    uint32_t h1 = 0, h2 = 0;
-                    for (int bb = 0; bb < chb; ++bb) {
-                        const uint4 w = *reinterpret_cast<const uint4*>(colx + (sgi + bb) * A.QS);
-                        h1 = __dp4a(w.x, 0x01010101u, h1);
-                        h1 = __dp4a(w.y, 0x01010101u, h1);
-                        h1 = __dp4a(w.z, 0x01010101u, h1);
-                        h1 = __dp4a(w.w, 0x01010101u, h1);
-                        h2 = __dp4a(w.x, w.x, h2);
-                        h2 = __dp4a(w.y, w.y, h2);
-                        h2 = __dp4a(w.z, w.z, h2);
-                        h2 = __dp4a(w.w, w.w, h2);
-                    }
-                    const uint4 bi = *reinterpret_cast<const uint4*>(colx + (sgi + chb) * A.QS);
-                    if (chr) {
-                        const uint32_t wv[4] = {bi.x, bi.y, bi.z, bi.w};
-#pragma unroll
-                        for (int m = 0; m < 4; ++m) {
-                            const int keep = min(max(chr - 4 * m, 0), 4);
-                            const uint32_t mk = keep == 4 ? 0xffffffffu : ((1u << (8 * keep)) - 1u);
-                            h1 = __dp4a(wv[m] & mk, 0x01010101u, h1);
-                            h2 = __dp4a(wv[m] & mk, wv[m], h2);
+                for (int is = 0; is < nr; is += A.VR) {
+                    const int ni = min(A.VR, nr - is);
+                    const int nseg = (ni + 15) >> 4;
+                    for (int task = tid; task < XW * nseg; task += kBT) {
+                        const int sgl = task / XW, x = task - sgl * XW;
+                        const int sgi = (is >> 4) + sgl, i0 = 16 * sgi;
+                        const uint8_t* colx = s_W + x * 16;
+                        const uint4 bo = *reinterpret_cast<const uint4*>(colx + sgi * A.QS);
+                        uint32_t h1 = 0, h2 = 0;
+                        for (int bb = 0; bb < chb; ++bb) {
+                            const uint4 w = *reinterpret_cast<const uint4*>(colx + (sgi + bb) * A.QS);
+                            h1 = __dp4a(w.x, 0x01010101u, h1);
+                            h1 = __dp4a(w.y, 0x01010101u, h1);
+                            h1 = __dp4a(w.z, 0x01010101u, h1);
+                            h1 = __dp4a(w.w, 0x01010101u, h1);
+                            h2 = __dp4a(w.x, w.x, h2);
+                            h2 = __dp4a(w.y, w.y, h2);
+                            h2 = __dp4a(w.z, w.z, h2);
+                            h2 = __dp4a(w.w, w.w, h2);
                         }
-                    }
-                    const uint32_t wo[4] = {bo.x, bo.y, bo.z, bo.w};
-                    const uint32_t wi[4] = {bi.x, bi.y, bi.z, bi.w};
-                    uint32_t* v1o = s_V1 + i0 * A.XV + x;
-                    uint32_t* v2o = s_V2 + i0 * A.XV + x;
+                        const uint4 bi = *reinterpret_cast<const uint4*>(colx + (sgi + chb) * A.QS);
+                        if (chr) {
+                            const uint32_t wv[4] = {bi.x, bi.y, bi.z, bi.w};
 #pragma unroll
-                    for (int u = 0; u < 16; ++u) {
-                        if (i0 + u < nr) {
-                            v1o[u * A.XV] = h1;
-                            v2o[u * A.XV] = h2;
-                            const uint32_t o = (wo[u >> 2] >> (8 * (u & 3))) & 0xffu;
-                            uint32_t in;
-                            if (chr == 0) {
-                                in = (wi[u >> 2] >> (8 * (u & 3))) & 0xffu;
-                            } else {
-                                const int R = i0 + u + ch;
-                                in = colx[(R >> 4) * A.QS + (R & 15)];
+                            for (int m = 0; m < 4; ++m) {
+                                const int keep = min(max(chr - 4 * m, 0), 4);
+                                const uint32_t mk = keep == 4 ? 0xffffffffu : ((1u << (8 * keep)) - 1u);
+                                h1 = __dp4a(wv[m] & mk, 0x01010101u, h1);
+                                h2 = __dp4a(wv[m] & mk, wv[m], h2);
                             }
-                            h1 = h1 + in - o;
-                            h2 = h2 + in * in - o * o;
+                        }
+                        const uint32_t wo[4] = {bo.x, bo.y, bo.z, bo.w};
+                        const uint32_t wi[4] = {bi.x, bi.y, bi.z, bi.w};
+                        uint32_t* v1o = s_V1 + 16 * sgl * A.XV + x;
+                        uint32_t* v2o = s_V2 + 16 * sgl * A.XV + x;
+#pragma unroll
+                        for (int u = 0; u < 16; ++u) {
+                            if (i0 + u < nr) {
+                                v1o[u * A.XV] = h1;
+                                v2o[u * A.XV] = h2;
+                                if (i0 + u + 1 == nr) {
+                                    s_L1[x] = h1;
+                                    s_L2[x] = h2;
+                                }
+                                const uint32_t o = (wo[u >> 2] >> (8 * (u & 3))) & 0xffu;
+                                uint32_t in;
+                                if (chr == 0) {
+                                    in = (wi[u >> 2] >> (8 * (u & 3))) & 0xffu;
+                                } else {
+                                    const int R = i0 + u + ch;
+                                    in = colx[(R >> 4) * A.QS + (R & 15)];
+                                }
+                                h1 = h1 + in - o;
+                                h2 = h2 + in * in - o * o;
+                            }
                         }
                     }
+                    bar_box();
+                    // S[j][i] = sums of V[i][j .. j + cw - 1]: a task is a row i and 16 columns j.
+                    const int jseg = (nc + 15) >> 4;
+                    const bool vec = (cw & 3) == 0;
+                    for (int task = tid; task < ni * jseg; task += kBT) {
+                        const int sg = task / ni, il = task - sg * ni, i = is + il;
+                        const int j0 = 16 * sg;
+                        const uint32_t* r1 = s_V1 + il * A.XV;
+                        const uint32_t* r2 = s_V2 + il * A.XV;
+                        uint32_t g1 = 0, g2 = 0;
+                        int bb = 0;
+                        for (; bb + 4 <= cw; bb += 4) {
+                            const uint4 v = *reinterpret_cast<const uint4*>(r1 + j0 + bb);
+                            const uint4 w = *reinterpret_cast<const uint4*>(r2 + j0 + bb);
+                            g1 += (v.x + v.y) + (v.z + v.w);
+                            g2 += (w.x + w.y) + (w.z + w.w);
+                        }
+                        for (; bb < cw; ++bb) {
+                            g1 += r1[j0 + bb];
+                            g2 += r2[j0 + bb];
+                        }
+#pragma unroll
+                        for (int u4 = 0; u4 < 16; u4 += 4) {
+                            const uint4 o1 = *reinterpret_cast<const uint4*>(r1 + j0 + u4);
+                            const uint4 o2 = *reinterpret_cast<const uint4*>(r2 + j0 + u4);
+                            uint4 i1, i2;
+                            if (vec) {
+                                i1 = *reinterpret_cast<const uint4*>(r1 + j0 + u4 + cw);
+                                i2 = *reinterpret_cast<const uint4*>(r2 + j0 + u4 + cw);
+                            } else {
+                                const uint32_t* p1 = r1 + j0 + u4 + cw;
+                                const uint32_t* p2 = r2 + j0 + u4 + cw;
+                                i1 = make_uint4(p1[0], p1[1], p1[2], p1[3]);
+                                i2 = make_uint4(p2[0], p2[1], p2[2], p2[3]);
+                            }
+                            const uint32_t oo1[4] = {o1.x, o1.y, o1.z, o1.w}, ii1[4] = {i1.x, i1.y, i1.z, i1.w};
+                            const uint32_t oo2[4] = {o2.x, o2.y, o2.z, o2.w}, ii2[4] = {i2.x, i2.y, i2.z, i2.w};
+#pragma unroll
+                            for (int m = 0; m < 4; ++m) {
+                                const int j = j0 + u4 + m;
+                                if (j < nc) {
+                                    s_S1[j * A.NRS + i] = __uint2float_rn(g1);
+                                    s_S2[j * A.NRS + i] = g2;
+                                    g1 = g1 + ii1[m] - oo1[m];
+                                    g2 = g2 + ii2[m] - oo2[m];
+                                }
+                            }
+                        }
+                    }
+                    if (is + ni < nr) bar_box();
                 }
-                asm volatile("bar.sync 1, %0;" ::"r"(kBT) : "memory");
-                box_rows(0, nr);
             }
         }
         held = true;
-        h_wr = win_r;
-        h_wc = win_c;
-        h_ch = ch;
-        h_cw = cw;
-        h_nr = nr;
-        h_nc = nc;
-        TC_PHASE(6)
-        bool ok = tc::mbar_wait(&s_mbar, phase, kTcWaitPolls);
+        TC_PHASE(4)
+        // One warp polls for the products, the others wait for it at the barrier. It first makes the
+        // bound of the estimates' error (below).
+        bool ok = true;
+        if (warp == 7) {
+            const float u24 = 6.0200e-08f;  // 1.01 x 2^-24
+            const float kz = sqrtf(pow2 ? __ull2float_rn(nsq) : static_cast<float>(out.sq) * nnf);
+            const float kc = sqrtf(nnf * (pow2 ? __uint2float_rn(c2)
+                                               : static_cast<float>(out.sq + out.csum * out.mean)));
+            if (lane == 0)
+                s_bu = A.measure == AR_NCC ? u24 * sqrtf(nnf) * (20.0f * kz + 5.0f * kc)
+                                           : u24 * (3400.0f * kz + 160.0f * kc);
+            ok = tc::mbar_wait(&s_mbar, phase, kTcWaitPolls);
+        }
         phase ^= 1u;
-        if (__syncthreads_or(!ok)) {
-            if (tid == 0) atomicExch(A.status, 1);
+        if (bar_main_or(!ok)) {
             failed = true;
+            mb ^= 1;  // this point's barrier with the patch warp is past
             break;
         }
         tc::fence_after_sync();
-        TC_PHASE(7)
+        if (tid == 0) tc::mbar_arrive(&s_free);
+        TC_PHASE(5)
 
-        // Pass 1: numerators out of Tensor Memory (one 16x256b read per warp), box sums from
-        // shared memory; estimates and upper bounds stay in registers. Value v
-        // of a thread is surface row i = 32 half + 8 (v / 4) + 2 (lane % 4) + v % 2, column
-        // j = 16 quarter + lane / 4 (+ 8 when v % 4 >= 2).
-        const float kk = __double2float_rn(
-            A.measure == AR_NCC ? __drcp_rn(__dmul_rn(cnorm, nn))
-                                : __drcp_rn(__dmul_rn(cnorm, __dsqrt_rn(nn))));
-        const float kk7 = 4.172325134277344e-07f * kk;  // 7u k
-        const float nnf = static_cast<float>(nnl);
-        const float csf = static_cast<float>(csum_d);
+        // Pass 1: numerators out of Tensor Memory (one 16x256b read per warp and accumulator), box
+        // sums from shared memory. Value v of a thread is surface row
+        // i = 32 half + 8 (v / 4) + 2 (lane % 4) + v % 2, column j = 16 quarter + lane / 4 (+ 8
+        // when v % 4 >= 2).
+        // The estimate of a value is nx r, with nx = nn D - sum(C) s1 and r the reciprocal root of
+        // its variance term vx = nn s2 - s1^2 (s2 for NCC), all in Float32: the value times
+        // kz = cnorm sqrt(nn) (NCC: cnorm nn). r depends on the window alone, so it is kept in a
+        // ring beside s1 and s2 and made for new rows only; it is 0 where s2 is 0 (the value is
+        // 0) and NaN where tv = nn s2 + s1^2 is above 2^11 vx, whose value is always evaluated
+        // exactly. Errors (u = 2^-24): vx is within 3u tv of exact, so r is within 3080u of exact;
+        // D, sum(C) s1, nx and the product round once each. So an estimate is within
+        // 3100u |value| + 1.05u (nn D + sum(C) s1) r / kz of the value, and by Cauchy-Schwarz the
+        // second term is at most 2.1u T_c T with T_c = |C| / cnorm and T = sqrt(nn s2 / vx) <= 32 (1
+        // for NCC). `bu` is (3400u + 5u T_c T) kz, above that (with kc = sqrt(nn sum(C^2))): a value
+        // whose estimate is more than 2 bu below the largest one is below that one.
+        const float csf = pow2 ? __uint2float_rn(cs) : static_cast<float>(out.csum);
         const int quarter = warp & 3, half = warp >> 2;
-        const uint32_t col0 = 0u;  // surface row i is accumulator column i
         const int ib0 = 32 * half + 2 * (lane & 3);
         const int jb0 = 16 * quarter + (lane >> 2);
         uint32_t dv[16];
-        float upb[16];
-        uint32_t vm = 0u;
-        float lmax = -INFINITY;
-        if (32 * half < nr) {
-            const uint32_t base = taddr + (static_cast<uint32_t>(32 * quarter) << 16) + col0 +
+        float sum = 0.0f;
+        float own = -INFINITY, own2 = -INFINITY;  // this thread's two largest estimates
+        int at = 0;                               // the value of the largest
+        bool odd = false;                         // an estimate was not made
+        if (32 * half < nr && 16 * quarter < nc) {
+            const uint32_t base = taddr + (static_cast<uint32_t>(32 * quarter) << 16) +
                                   static_cast<uint32_t>(32 * half);
-            uint32_t dv1[kTc2Issuers - 1][16];
-            tc::tmem_ld16dp(base, dv);
+            {
+                // The issuers' shares.
+                uint32_t d1[16];
+                tc::tmem_ld16dp(base, dv);
+                tc::tmem_ld16dp(base + acc1, d1);
+                tc::tmem_wait_ld();
 #pragma unroll
-            for (int t = 1; t < kTc2Issuers; ++t) tc::tmem_ld16dp(base + static_cast<uint32_t>(t) * acc1, dv1[t - 1]);
-            tc::tmem_wait_ld();
+                for (int v = 0; v < 16; ++v) dv[v] += d1[v];
+                for (int s = 2; s < A.issuers; ++s) {
+                    tc::tmem_ld16dp(base + static_cast<uint32_t>(s) * acc1, d1);
+                    tc::tmem_wait_ld();
 #pragma unroll
-            for (int t = 1; t < kTc2Issuers; ++t)
+                    for (int v = 0; v < 16; ++v) dv[v] += d1[v];
+                }
+            }
+            clear_acc();  // for the next point (waited for before its products)
+            // Values v and v + 1 are surface rows i and i + 1 of one column (nr is even): estimated
+            // as a packed pair, from clamped indices so that all loads can be in flight.
+            int r0[4], r1[4];
 #pragma unroll
-                for (int v = 0; v < 16; ++v) dv[v] += dv1[t - 1][v];  // the issuers' shares
-            // Values v and v + 1 are surface rows i and i + 1 of one column: estimated as a pair.
+            for (int m = 0; m < 4; ++m) {
+                r0[m] = ring(min(ib0 + 8 * m, nr - 2));
+                r1[m] = r0[m] + 1 == A.NRS ? 0 : r0[m] + 1;
+            }
+            auto pair = [&](int m, int c, float2 s1, float2 r) {
+                const int v = 4 * m + 2 * c;
+                const float2 nx = __ffma2_rn(
+                    make_float2(nnf, nnf),
+                    make_float2(__uint2float_rn(dv[v]), __uint2float_rn(dv[v + 1])),
+                    neg2(__fmul2_rn(make_float2(csf, csf), s1)));
+                float2 e = __fmul2_rn(nx, r);
+                const bool in = jb0 + 8 * c < nc && ib0 + 8 * m < nr;
+                sum += in ? e.x + e.y : 0.0f;
+                e.x = in ? e.x : -INFINITY;
+                e.y = in ? e.y : -INFINITY;
+                own2 = fmaxf(own2, fminf(own, e.x));
+                at = e.x > own ? v : at;
+                own = fmaxf(own, e.x);
+                own2 = fmaxf(own2, fminf(own, e.y));
+                at = e.y > own ? v + 1 : at;
+                own = fmaxf(own, e.y);
+            };
+            if (carry) {
 #pragma unroll
-            for (int v = 0; v < 16; v += 2) {
-                const int i = ib0 + 8 * (v >> 2), j = jb0 + ((v & 2) ? 8 : 0);
-                upb[v] = upb[v + 1] = -INFINITY;
-                if (j < nc && i < nr) {
-                    const bool two = i + 1 < nr;
-                    vm |= (two ? 3u : 1u) << v;
-                    const int o = j * A.NRS + ring(i), o1 = j * A.NRS + ring(i + 1);
-                    const uint32_t b1 = two ? s_S1[o1] : 0u, b2 = two ? s_S2[o1] : 0u;
-                    float2 bnd;
-                    const float2 est = tc_estimate2(dv[v], dv[v + 1], s_S1[o], b1, s_S2[o], b2,
-                                                    nnf, csf, kk, kk7, A.measure, &bnd);
-                    upb[v] = est.x + bnd.x;
-                    lmax = fmaxf(lmax, est.x - bnd.x);
-                    if (two) {
-                        upb[v + 1] = est.y + bnd.y;
-                        lmax = fmaxf(lmax, est.y - bnd.y);
+                for (int c = 0; c < 2; ++c) {
+                    const float* S = s_S1 + min(jb0 + 8 * c, nc - 1) * A.NRS;
+                    const float* R = s_R + min(jb0 + 8 * c, nc - 1) * A.NRS;
+#pragma unroll
+                    for (int m = 0; m < 4; ++m)
+                        pair(m, c, make_float2(S[r0[m]], S[r1[m]]), make_float2(R[r0[m]], R[r1[m]]));
+                }
+            } else {
+                // Every row is new: the reciprocal roots are made here, by all warps.
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const int o = min(jb0 + 8 * c, nc - 1) * A.NRS;
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) {
+                        const float2 s1 = make_float2(s_S1[o + r0[m]], s_S1[o + r1[m]]);
+                        const float2 r = make_float2(recip(s1.x, s_S2[o + r0[m]]), recip(s1.y, s_S2[o + r1[m]]));
+                        s_R[o + r0[m]] = r.x;
+                        s_R[o + r1[m]] = r.y;
+                        pair(m, c, s1, r);
                     }
                 }
             }
+            odd = isnan(sum);
+        } else {
+            clear_acc();
+#pragma unroll
+            for (int v = 0; v < 16; ++v) dv[v] = 0u;
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) lmax = fmaxf(lmax, __shfl_xor_sync(kFull, lmax, o));
-        if (lane == 0) s_fmax[warp] = lmax;
-        if (tid == 0) s_ncand = 0;
-        __syncthreads();
-        TC_PHASE(8)
-        float M = s_fmax[0];
-        for (int w = 1; w < kTcThreads / 32; ++w) M = fmaxf(M, s_fmax[w]);
-        // Pass 2: values whose upper bound reaches M (or whose estimate was not made) go to a
-        // list and are normalised exactly, one per thread.
-#pragma unroll
-        for (int v = 0; v < 16; ++v) {
-            if (((vm >> v) & 1u) && (upb[v] >= M || isnan(upb[v]))) {
-                const int c = atomicAdd(&s_ncand, 1);
-                s_num[c] = dv[v];
-                s_cI[c] = (static_cast<uint32_t>(ib0 + 8 * (v >> 2) + (v & 1)) << 16) |
-                          static_cast<uint32_t>(jb0 + ((v & 2) ? 8 : 0));
+        // The warp's largest estimate, where it is, and the largest of its others (+inf when some
+        // estimate was not made).
+        {
+            const float top = warp_max(own);
+            const unsigned who = __ballot_sync(kFull, own == top && own > -INFINITY);
+            const int first = who ? __ffs(who) - 1 : 0;
+            const float sec = warp_max(odd ? INFINITY : lane == first ? own2 : own);
+            if (lane == first) {
+                s_top[warp] = top;
+                s_sec[warp] = sec;
+                s_at[warp] = ((ib0 + 8 * (at >> 2) + (at & 1)) << 16) | (jb0 + ((at & 2) ? 8 : 0));
             }
         }
-        __syncthreads();
-        const int ncand = s_ncand;
-        unsigned rm = 0;
-        float pv = 0.0f;
+        tc::fence_before_sync();
+        bar_main();  // also: the accumulators are read
+        tc::fence_after_sync();
+        TC_PHASE(6)
+        // Lane w looks at warp w's: is the largest estimate more than the bound above every other?
         int pi = 0, pj = 0;
-        if (ncand == 1 && M > -INFINITY) {
-            // M is finite, so the value whose lower bound is M is in the list; when it is the
-            // only entry, every other FP32 surface value is at most its upper bound, below M,
-            // and this one is at least M: it is the strict (so the first) maximum.
-            pi = static_cast<int>(s_cI[0] >> 16);
-            pj = static_cast<int>(s_cI[0] & 0xFFFFu);
+        const float wt = lane < 8 ? s_top[lane] : -INFINITY;
+        const float M = warp_max(wt);
+        const float cut = M - 2.0f * s_bu;
+        const int mw = __ffs(__ballot_sync(kFull, wt == M)) - 1;
+        const bool unique =
+            M > -INFINITY &&
+            !__any_sync(kFull, lane < 8 && (!(s_sec[lane & 7] < cut) || (lane != mw && !(wt < cut))));
+        if (unique && !A.surf_out) {
+            // Every other value is below this one: it is the strict (so the first) maximum.
+            pi = s_at[mw] >> 16;
+            pj = s_at[mw] & 0xFFFF;
         } else {
+            // Pass 2: the values whose estimate is within the bounds of M (or was not made), exactly,
+            // from the numerators in shared memory (in place of the operands).
+            const double nn = static_cast<double>(nnl);
+            double mean = out.mean, sq = out.sq;
+            if (pow2) tc2_chip_stats(nnl, cs, c2, &mean, &sq);
+            const double cnorm = __dsqrt_rn(sq);
+#pragma unroll
+            for (int v = 0; v < 16; ++v) {
+                const int i = ib0 + 8 * (v >> 2) + (v & 1), j = jb0 + ((v & 2) ? 8 : 0);
+                if (i < nr && j < nc) s_num[j * A.NRS + i] = dv[v];
+            }
+            bar_main();
             unsigned long long best = 0ull;
-            for (int c = tid; c < ncand; c += bd) {
-                const int i = static_cast<int>(s_cI[c] >> 16), j = static_cast<int>(s_cI[c] & 0xFFFFu);
+            for (int e = tid; e < nr * nc; e += kTcThreads) {
+                const int j = e / nr, i = e - j * nr;
                 const int o = j * A.NRS + ring(i);
-                const float x = tc_exact(s_num[c], s_S1[o], s_S2[o], mean, nn, cnorm, A.measure);
+                const uint32_t D = s_num[j * A.NRS + i], s2 = s_S2[o];
+                const float s1 = s_S1[o];
+                if (__fmaf_rn(nnf, __uint2float_rn(D), -__fmul_rn(csf, s1)) * s_R[o] < cut && !A.surf_out) continue;
+                const float x = tc2_exact(D, s1, s2, mean, nn, cnorm, A.measure);
                 const unsigned long long key = argmax_key(x, static_cast<unsigned>(i * nc + j));
                 best = key > best ? key : best;
+                if (A.surf_out) A.surf_out[k * static_cast<int64_t>(A.NRM) * A.NCM + e] = x;
             }
-            best = block_max_u64(best, reinterpret_cast<unsigned long long*>(s_red));
+            best = block_max_u64<true>(best, reinterpret_cast<unsigned long long*>(s_red));
+            unsigned rm = 0;
+            float pv = 0.0f;
             if (key_decode(best, &rm, &pv)) {
                 pi = static_cast<int>(rm / nc);
                 pj = static_cast<int>(rm % nc);
             }
+            bar_main();  // s_num and s_red are read
         }
-        TC_PHASE(9)
+        TC_PHASE(7)
         if (A.flops && tid == 0)
-            atomicAdd(A.flops, 2ull * static_cast<unsigned long long>(ch) * cw * nr * nc);
-        if (A.surf_out) {
-            // Every value exactly (diagnostic surfaces): numerators to shared memory first.
-#pragma unroll
-            for (int v = 0; v < 16; ++v)
-                if ((vm >> v) & 1u)
-                    s_num[(jb0 + ((v & 2) ? 8 : 0)) * A.NRS + ib0 + 8 * (v >> 2) + (v & 1)] = dv[v];
-            __syncthreads();
-            float* so = A.surf_out + k * static_cast<int64_t>(A.NRM) * A.NCM;
-            for (int e = tid; e < nr * nc; e += bd) {
-                const int o = (e / nr) * A.NRS + (e % nr), os = (e / nr) * A.NRS + ring(e % nr);
-                so[e] = tc_exact(s_num[o], s_S1[os], s_S2[os], mean, nn, cnorm, A.measure);
-            }
-        }
+            atomicAdd(A.flops, 2ull * static_cast<unsigned long long>(nnl) * nr * nc);
+        // The peak's or the patch's numerators and sums, to the helper.
         const bool single = A.up == 1 || nr < 5 || nc < 5;
         const int pi0 = single ? pi : min(max(pi - 2, 0), max(nr - 5, 0));
         const int pj0 = single ? pj : min(max(pj - 2, 0), max(nc - 5, 0));
         const int span = single ? 1 : 5;
+        if (pi0 < 32 * half + 32 && pi0 + span > 32 * half && pj0 < 16 * quarter + 16 &&
+            pj0 + span > 16 * quarter) {
 #pragma unroll
-        for (int v = 0; v < 16; ++v) {
-            const int a = ib0 + 8 * (v >> 2) + (v & 1) - pi0, b = jb0 + ((v & 2) ? 8 : 0) - pj0;
-            if (a >= 0 && a < span && b >= 0 && b < span && ((vm >> v) & 1u)) s_pd[b * 5 + a] = dv[v];
-        }
-        __syncthreads();
-        if (single) {
-            if (tid == 0) {
-                A.out.dx[k] = __double2float_rn(
-                    __dadd_rn(static_cast<double>(pj - static_cast<int>(prx)), A.pts.dx0[k]));
-                A.out.dy[k] = __double2float_rn(
-                    __dadd_rn(static_cast<double>(pi - static_cast<int>(pry)), A.pts.dy0[k]));
-                const int o = pj * A.NRS + ring(pi);
-                A.out.corr[k] = tc_exact(s_pd[0], s_S1[o], s_S2[o], mean, nn, cnorm, A.measure);
-            }
-        } else {
-            const int slot = s_slot;
-            if (tid < 25) {
-                const int a = tid % 5, b = tid / 5;
-                const int o = (pj0 + b) * A.NRS + ring(pi0 + a);
-                A.sub_patch[static_cast<int64_t>(slot) * 25 + tid] =
-                    tc_exact(s_pd[tid], s_S1[o], s_S2[o], mean, nn, cnorm, A.measure);
-            }
-            if (tid == 0) {
-                A.sub_point[slot] = k;
-                A.sub_origin[2 * slot] = pi0;
-                A.sub_origin[2 * slot + 1] = pj0;
+            for (int v = 0; v < 16; ++v) {
+                const int i = ib0 + 8 * (v >> 2) + (v & 1), j = jb0 + ((v & 2) ? 8 : 0);
+                const unsigned a = static_cast<unsigned>(i - pi0), c = static_cast<unsigned>(j - pj0);
+                if (a < static_cast<unsigned>(span) && c < static_cast<unsigned>(span)) {  // inside the surface
+                    const int o = j * A.NRS + ring(i);
+                    out.D[c * 5 + a] = dv[v];
+                    out.s1[c * 5 + a] = s_S1[o];
+                    out.s2[c * 5 + a] = s_S2[o];
+                }
             }
         }
-        TC_PHASE(10)
+        if (tid == 0) {
+            out.kind = single ? 1 : 2;
+            out.pi = pi0;
+            out.pj = pj0;
+        }
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&s_outb[mb]);
+        mb ^= 1;
+        TC_PHASE(8)
         TC_PHASE_POINT
     }
     TC_PHASE_FLUSH
-#ifdef AR_TC_PHASES
-    if (tid == kTcThreads - 32) {
-        atomicAdd(&g_tc_phase[12], tmi_issue);
-        atomicAdd(&g_tc_phase[13], tmi_done);
+    if (failed) {
+        if (tid == 0) atomicExch(A.status, 1);
+        // Products may still be in flight: a bounded time before the accumulators are freed.
+        tc::mbar_wait(&s_mbar, phase ^ 1u, kTcWaitPolls);
     }
-#endif
-    if (failed) tc::mbar_wait(&s_mbar, phase ^ 1u, kTcWaitPolls);
+    tc::tmem_wait_st();
+    if (tid == 0) s_more[mb] = 0;
+    bar_products();
+    }
     tc::fence_before_sync();
     __syncthreads();
     if (warp == 0) tc::tmem_dealloc(taddr, A.tmem_cols);
@@ -3355,14 +3669,6 @@ __device__ __forceinline__ void warp_best(float& bv, int& bi) {
     }
 }
 
-// Largest value of a warp (no lane NaN): floats as ordered integers, one reduction instruction.
-__device__ __forceinline__ float warp_max(float v) {
-    int i = __float_as_int(v);
-    i ^= (i >> 31) & 0x7fffffff;
-    i = __reduce_max_sync(kFull, i);
-    return __int_as_float(i ^ ((i >> 31) & 0x7fffffff));
-}
-
 // A region of a level: rows r0 .. and columns c0 .. stored column-major with leading dimension
 // kZR from `p`.
 struct Region {
@@ -3803,6 +4109,7 @@ size_t tmem_smem_floor(uint32_t cols, size_t static_smem) {
 struct TcPlan {
     int NB, QM, QS, PS, PC, XS, XT, NRS, NRM, NCM, CHM, CWM, BC, big, MT;
     unsigned off_E, off_W, off_T, off_P, off_V, off_S1, off_S2, off_num, off_est, off_red;
+    unsigned off_L = 0, off_rawW = 0, off_rawC = 0;
     int XV = 0, VR = 0, acc1_col = 0, issuers = 2;
     uint32_t tmem_cols;
     size_t smem;
@@ -3811,6 +4118,9 @@ struct TcPlan {
 // Shared-memory and Tensor Memory plan of k_corr_tc2 for a pass's largest geometry; false when
 // the pass does not fit it (surfaces beyond 64 x 64, chip operand larger than shared memory,
 // accumulator beyond 512 columns).
+// Dynamic shared memory that leaves room for two CTAs (228 KB per SM, less 1 KB and the static
+// shared memory of each).
+constexpr size_t kTc2TwoCtas = 110 * 1024;
 bool plan_corr_tc2(const PassGeometry& g, size_t smem_cap, TcPlan* P) {
     const int ch = static_cast<int>(g.max_ch), cw = static_cast<int>(g.max_cw);
     const int nr = static_cast<int>(g.max_nr), nc = static_cast<int>(g.max_nc);
@@ -3830,39 +4140,55 @@ bool plan_corr_tc2(const PassGeometry& g, size_t smem_cap, TcPlan* P) {
     P->PC = round_up(kPadL + P->NB + 20, 16);
     P->NRS = nr | 1;
     P->XV = round_up(cw + nc - 1, 32) + 4;
-    // kTc2Issuers accumulators whose column i is surface row i (the products write columns below
-    // round16(nr), the epilogue reads 32 columns per half of the surface rows).
-    const int stride = nr > 32 ? 64 : 32;
-    uint32_t t1 = 32;
-    while (static_cast<int>(t1) < kTc2Issuers * stride) t1 <<= 1;
-    P->acc1_col = stride;
-    P->tmem_cols = t1;
+    // Four accumulators of 64 or 32 columns, each with an issuing thread (column i is surface row
+    // i: the products write columns below round16(nr), the epilogue reads 32 columns per half of
+    // the surface rows).
+    P->acc1_col = nr > 32 ? 64 : 32;
+    P->issuers = 4;
+    P->tmem_cols = static_cast<uint32_t>(4 * P->acc1_col);
     auto a16 = [](size_t v) { return (v + 15) & ~size_t(15); };
     const size_t Eb = static_cast<size_t>(cw) * P->PS;
     const size_t Wb = static_cast<size_t>(P->QM) * P->QS;
     const size_t Pb = a16(static_cast<size_t>(cw) * P->PC);
-    const size_t Vb = a16(2 * (static_cast<size_t>(nr) * P->XV + 16) * 4);
     const size_t nbytes = a16(static_cast<size_t>(nc) * P->NRS * 4);
-    // [E][W][P][V1, V2 | candidate numerators and indices][S1][S2][red]
+    const size_t rawW = static_cast<size_t>(cw + nc - 1) * (P->QM + 1) * 16;
+    const size_t rawC = 2 * static_cast<size_t>(cw) * ((ch + 15) / 16 + 1) * 16;
+    // [E][W][V1, V2 | raw window, raw chip and mask][P][S1][S2][R][L1, L2][red]; every value's numerator
+    // takes E and W's place once the products are done. V holds the column sums of `vr` surface
+    // rows.
+    auto layout = [&](int vr) {
+        P->VR = vr;
+        size_t off = 0;
+        P->off_E = P->off_num = 0;
+        off += Eb;
+        P->off_W = static_cast<unsigned>(off);
+        off = std::max(off + Wb, nbytes);
+        P->off_V = P->off_rawW = static_cast<unsigned>(off);
+        P->off_rawC = static_cast<unsigned>(off + rawW);
+        off += std::max(a16(2 * (static_cast<size_t>(vr) * P->XV + 16) * 4), rawW + rawC);
+        P->off_P = static_cast<unsigned>(off);
+        off += Pb;
+        P->off_S1 = static_cast<unsigned>(off);
+        off += nbytes;
+        P->off_S2 = static_cast<unsigned>(off);
+        off += nbytes;
+        P->off_est = static_cast<unsigned>(off);
+        off += nbytes;
+        P->off_L = static_cast<unsigned>(off);
+        off += a16(2 * static_cast<size_t>(P->XV) * 4);
+        P->off_red = static_cast<unsigned>(off);
+        return off + 3 * 32 * 8;
+    };
+    // As many rows of V as leave room for two CTAs per SM (every one of them, else multiples of
+    // 16); where not even 16 do, as many as fit one.
     size_t off = 0;
-    P->off_E = 0;
-    off += Eb;
-    P->off_W = static_cast<unsigned>(off);
-    off += Wb;
-    P->off_P = static_cast<unsigned>(off);
-    off += Pb;
-    P->off_V = static_cast<unsigned>(off);
-    P->off_num = P->off_V;
-    P->off_est = static_cast<unsigned>(off + nbytes);
-    // The region also takes the window's raw 16-byte chunks before the box sums.
-    const size_t rawb = static_cast<size_t>(P->XS) * (P->QM + 1) * 16;
-    off += std::max(std::max(Vb, 2 * nbytes), rawb);
-    P->off_S1 = static_cast<unsigned>(off);
-    off += nbytes;
-    P->off_S2 = static_cast<unsigned>(off);
-    off += nbytes;
-    P->off_red = static_cast<unsigned>(off);
-    off += 3 * 32 * 8;
+    for (size_t cap : {kTc2TwoCtas, smem_cap}) {
+        cap = std::min(cap, smem_cap);
+        int vr = nr;
+        off = layout(vr);
+        while (off > cap && vr > 16) off = layout(vr = std::max(16, (vr - 1) & ~15));
+        if (off <= cap) break;
+    }
     P->off_T = 0;
     P->BC = cw;
     P->big = 0;
@@ -4490,6 +4816,9 @@ cudaError_t launch_track_impl(int dtype, const void* ref, const void* sec, const
         B.off_num = TP.off_num;
         B.off_est = TP.off_est;
         B.off_red = TP.off_red;
+        B.off_L = TP.off_L;
+        B.off_rawW = TP.off_rawW;
+        B.off_rawC = TP.off_rawC;
         B.XV = TP.XV;
         B.acc1_col = TP.acc1_col;
         B.issuers = TP.issuers;
@@ -4524,7 +4853,7 @@ cudaError_t launch_track_impl(int dtype, const void* ref, const void* sec, const
         if (e != cudaSuccess) return e;
         const int grid = static_cast<int>(
             std::max<int64_t>(1, std::min<int64_t>(pts.n, static_cast<int64_t>(num_sms) * per_sm_tc)));
-        kern<<<grid, kTcThreads, tc_smem, stream>>>(B);
+        kern<<<grid, tc2 ? kTc2Threads : kTcThreads, tc_smem, stream>>>(B);
         e = cudaGetLastError();
             return e;
     };
