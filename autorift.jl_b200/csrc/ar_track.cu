@@ -634,6 +634,692 @@ __global__ void __launch_bounds__(kCorrThreads, 2) k_corr(const CorrArgs A) {
     }
 }
 
+// Optional phase timer (compiled in with -DAR_TC_PHASES, for profiling builds only): thread 0
+// of each CTA accumulates clock64() cycles between the marks below, per phase, and adds them to
+// g_tc_phase at exit; entry 15 counts the points that reached the output phase.
+#ifdef AR_TC_PHASES
+__device__ unsigned long long g_tc_phase[16];
+#define TC_PHASE_INIT unsigned long long tcp_t = clock64(), tcp_acc[12] = {}, tcp_n = 0;
+#define TC_PHASE(n)                              \
+    if (tid == 0) {                              \
+        const unsigned long long t_ = clock64(); \
+        tcp_acc[n] += t_ - tcp_t;                \
+        tcp_t = t_;                              \
+    }
+#define TC_PHASE_POINT \
+    if (tid == 0) ++tcp_n;
+#define TC_PHASE_FLUSH                                                           \
+    if (tid == 0) {                                                              \
+        for (int n_ = 0; n_ < 12; ++n_) atomicAdd(&g_tc_phase[n_], tcp_acc[n_]); \
+        atomicAdd(&g_tc_phase[15], tcp_n);                                       \
+    }
+#else
+#define TC_PHASE_INIT
+#define TC_PHASE(n)
+#define TC_PHASE_POINT
+#define TC_PHASE_FLUSH
+#endif
+
+// ----------------------------------------------------------------------------------------------
+// Direct FP32 correlation of UInt16, Int16 and Float32 imagery and of turned chips of any type,
+// surfaces of one tile (k_corr_fp). The same numerator as k_corr, product for product: FP32 over
+// two chip columns in the same order, then FP64; but
+//  * two surface columns per thread as packed FP32 pairs: the window is staged as pairs
+//    (W[r, x], W[r, x + 1]), so one 64-bit load feeds a packed FMA whatever the row, and a product
+//    pair costs one issue slot;
+//  * even and odd window columns lie in separate halves, so that lanes on consecutive column pairs
+//    read rows WS pairs apart (WS odd: 16 of them conflict-free), and the lanes take 16 column
+//    pairs of a row group at a time as far as these go;
+//  * where the column pairs and row groups do not fill the block, the chip's columns are split over
+//    the free threads (whole two-column groups; the FP64 sums are added at the end);
+//  * box sums from column sums of a few rows at a time, instead of tables of every window row, with
+//    counts of non-zero values beside them, so that windows of zeros keep exactly zero variance;
+//    each point's variance terms are kept (8 bytes a value), not its sums, and serve every angle of
+//    an integer image;
+//  * Float32 estimates of the surface, with the FP64 normalisation (src/correlate.jl:591-600) for
+//    the candidates of the maximum and the patch only.
+// Bound: the FMA pipe takes two cycles for a packed warp instruction, 20.5 k cycles a point at chip
+// 32 / radius 25 of the 46 k a point takes (30 k of products per CTA without a neighbour; the box
+// sums, the window and the estimates around them are FP64 and load latency, which the other of
+// the two CTAs per SM covers only in part). Measured, chip 32 / radius 25, against k_corr on the
+// same pass: Float32 (14.6 k points) 3.00 -> 2.52 ms, UInt16 2.99 -> 2.50 ms, three angles on UInt8
+// 11.84 -> 6.24 ms; chip 16 / radius 10 0.94 -> 0.85 ms; chip 48 / radius 30 5.08 -> 4.54 ms.
+// Surfaces of more than one tile stay with k_corr.
+
+// A pixel with zero padding from an address that is always valid, so that loads need no branch and
+// several can be in flight.
+template <typename T>
+__device__ __forceinline__ T pixel_at(const T* img, int64_t nrows, int64_t ncols, int64_t r, int64_t c) {
+    const int64_t rr = min(max(r, static_cast<int64_t>(0)), nrows - 1);
+    const int64_t cc = min(max(c, static_cast<int64_t>(0)), ncols - 1);
+    const T v = img[rr + cc * nrows];
+    return r == rr && c == cc ? v : T(0);
+}
+
+// rotated_sample from the chip staged in shared memory (column b at raw + b * stride).
+__device__ __forceinline__ float rotated_at(const float* raw, int stride, int ch, int cw, int a, int b,
+                                            double sn, double cs) {
+    const double yc = static_cast<double>(ch + 1) * 0.5, xc = static_cast<double>(cw + 1) * 0.5;
+    const double dy = static_cast<double>(a + 1) - yc, dx = static_cast<double>(b + 1) - xc;
+    const double sy = __dadd_rn(__dadd_rn(yc, __dmul_rn(cs, dy)), __dmul_rn(sn, dx));
+    const double sx = __dadd_rn(__dsub_rn(xc, __dmul_rn(sn, dy)), __dmul_rn(cs, dx));
+    const double fi = floor(sy), fj = floor(sx);
+    const bool in = fi >= 1.0 && fj >= 1.0 && fi + 1.0 <= static_cast<double>(ch) &&
+                    fj + 1.0 <= static_cast<double>(cw);
+    const int i0 = in ? static_cast<int>(fi) : 1, j0 = in ? static_cast<int>(fj) : 1;  // 1-based
+    // An even chip side has a second row and column, so the clamped indices are in the chip too.
+    const float* q = raw + (j0 - 1) * stride + i0 - 1;
+    const float p00 = q[0], p10 = q[1], p01 = q[stride], p11 = q[stride + 1];
+    const double fy = __dsub_rn(sy, fi), fx = __dsub_rn(sx, fj);
+    const double gx = __dsub_rn(1.0, fx), gy = __dsub_rn(1.0, fy);
+    const double top = __dadd_rn(__dmul_rn(gx, static_cast<double>(p00)), __dmul_rn(fx, static_cast<double>(p01)));
+    const double bot = __dadd_rn(__dmul_rn(gx, static_cast<double>(p10)), __dmul_rn(fx, static_cast<double>(p11)));
+    return in ? __double2float_rn(__dadd_rn(__dmul_rn(gy, top), __dmul_rn(fy, bot))) : 0.0f;
+}
+
+__device__ __noinline__ float fp_exact(double num, double wvar, double cnorm) {
+    const double den = __dmul_rn(cnorm, __dsqrt_rn(wvar));
+    return den > 0.0 ? __double2float_rn(__ddiv_rn(num, den)) : 0.0f;
+}
+
+template <typename T, bool ROT>
+__global__ void __launch_bounds__(kCorrThreads, 2) k_corr_fp(const CorrArgs A) {
+    typedef Traits<T> Tr;
+    extern __shared__ __align__(16) unsigned char smem[];
+    float* s_chip = reinterpret_cast<float*>(smem);
+    float2* s_win = reinterpret_cast<float2*>(smem + A.off_win);
+    // Partial sums, after the products: in the window's place, or beside it where it stays.
+    double* s_ex = reinterpret_cast<double*>(smem + A.off_surf2);
+    // Box sums: exact integers for integer types (below 2^32 for UInt8), else FP64.
+    typedef typename std::conditional<
+        sizeof(T) == 1, uint32_t, typename std::conditional<Tr::integer, long long, double>::type>::type BS;
+    BS* s_v1 = reinterpret_cast<BS*>(smem + A.off_ph1);
+    BS* s_v2 = s_v1 + kCorrThreads * A.TI;
+    float* s_raw = reinterpret_cast<float*>(smem + A.off_surf);  // rotation search: the chip itself
+    double* s_wv = reinterpret_cast<double*>(smem + A.off_ph2);
+    double* s_red = reinterpret_cast<double*>(smem + A.off_red);
+    __shared__ long long s_field[2][8];
+    __shared__ float s_top[kCorrThreads / 32], s_sec[kCorrThreads / 32];
+    __shared__ int s_at[kCorrThreads / 32];
+    __shared__ double s_pn[25], s_pw[25];  // the patch's numerators and variance terms
+    __shared__ float s_pp[25], s_best[25];  // its values, and the best angle's
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int nwarps = kCorrThreads / 32;
+    const T* ref = static_cast<const T*>(A.ref);
+    const T* sec = static_cast<const T*>(A.sec);
+    const int64_t NR = A.nrows + 2 * A.pady, NC = A.ncols + 2 * A.padx;
+    const double shx = static_cast<double>(A.padx) + 0.5;
+    const double shy = static_cast<double>(A.pady) + 0.5;
+
+    // The next point's eight fields, copied into shared memory a point ahead.
+    auto prefetch = [&](int64_t k, int b) {
+        if (tid < 8 && k < A.pts.n) {
+            const void* f[8] = {A.pts.x, A.pts.y, A.pts.rx, A.pts.ry, A.pts.dx0, A.pts.dy0, A.pts.csx, A.pts.csy};
+            const void* src = f[0];
+#pragma unroll
+            for (int q = 1; q < 8; ++q) src = tid == q ? f[q] : src;
+            tc::cp_async8(&s_field[b][tid], static_cast<const char*>(src) + 8 * k);
+        }
+        tc::cp_async_commit();
+    };
+    prefetch(blockIdx.x, 0);
+    int fb = 0;
+    TC_PHASE_INIT
+    for (int64_t k = blockIdx.x; k < A.pts.n; k += gridDim.x, fb ^= 1) {
+        tc::cp_async_wait_all();
+        __syncthreads();  // the fields are here; buffers of the previous point are no longer read
+        prefetch(k + gridDim.x, fb ^ 1);
+        const long long* fld = s_field[fb];
+        const int64_t prx = fld[2], pry = fld[3], csx = fld[6], csy = fld[7];
+        const double px0 = __longlong_as_double(fld[0]), py0 = __longlong_as_double(fld[1]);
+        const double dx0 = __longlong_as_double(fld[4]), dy0 = __longlong_as_double(fld[5]);
+        if (!(prx > 0 && pry > 0)) continue;  // issearchable (src/points.jl:116-117)
+
+        // Geometry in padded 1-based coordinates (src/track.jl:207-210, src/points.jl:358-395).
+        const double xs = px0 + shx, ys = py0 + shy;
+        const int64_t hx = csx / 2, hy = csy / 2;
+        const int64_t ccx = static_cast<int64_t>(floor(__dsub_rn(xs, dx0)));
+        const int64_t ccy = static_cast<int64_t>(floor(__dsub_rn(ys, dy0)));
+        const int64_t wcx = static_cast<int64_t>(floor(xs)), wcy = static_cast<int64_t>(floor(ys));
+        const int64_t cr0 = ccy - hy, cr1 = ccy + hy - 1, cc0 = ccx - hx, cc1 = ccx + hx - 1;
+        const int64_t wr0 = wcy - hy - pry, wr1 = wcy + hy + pry - 2;
+        const int64_t wc0 = wcx - hx - prx, wc1 = wcx + hx + prx - 2;
+        // checkbounds (src/track.jl:271-272): an empty range is always in bounds.
+        const bool chip_in = (cr1 < cr0 || cc1 < cc0) ||
+                             (cr0 >= 1 && cr1 <= NR && cc0 >= 1 && cc1 <= NC);
+        const bool win_in = (wr1 < wr0 || wc1 < wc0) ||
+                            (wr0 >= 1 && wr1 <= NR && wc0 >= 1 && wc1 <= NC);
+        if (!chip_in || !win_in) continue;
+        const int ch = static_cast<int>(2 * hy), cw = static_cast<int>(2 * hx);
+        const int nr = static_cast<int>(2 * pry), nc = static_cast<int>(2 * prx);
+        if (ch <= 0 || cw <= 0) continue;  // an empty chip has no valid pixel
+        if (ch > A.CHP || cw > A.CWM || nr > A.NRS || nc > A.NCM) continue;  // not sized for
+        const int64_t chip_r = cr0 - 1 - A.pady, chip_c = cc0 - 1 - A.padx;
+        const int64_t win_r = wr0 - 1 - A.pady, win_c = wc0 - 1 - A.padx;
+        const int chp = (ch + kUA - 1) & ~(kUA - 1);
+        const double nn = static_cast<double>(ch * cw);
+
+        // This thread's share of the products: column pair p, row group g, part `part` of the
+        // chip's columns.
+        const int npair = nc >> 1, ngrp = (nr + kMI - 1) / kMI, items = npair * ngrp;
+        int split = 1;
+        while (2 * split * items <= kCorrThreads && 4 * split <= cw && split < 8) split *= 2;
+        const int part = tid / items, it = tid - part * items;
+        const int npf = npair & ~15, itr = it - npf * ngrp, npr = max(npair - npf, 1);
+        const int g = itr < 0 ? it / npf : itr / npr;
+        const int p = itr < 0 ? it - g * npf : npf + itr - g * npr, il = g * kMI;
+        const bool active = part < split;
+        const int XW = cw + nc - 1, XH = (A.CWM + A.NCM) >> 1;
+
+        const int nang = ROT ? A.rot.count : 1;
+        float bestpk = -INFINITY;
+        bool found = false, have_var = false, skip = false, staged = false;
+        float staged_cs = 0.0f;
+        int pi0 = 0, pj0 = 0;
+        const bool single = A.up == 1 || nr < 5 || nc < 5;
+        for (int ia = 0; ia < nang; ++ia) {
+            const bool turn = ROT && A.rot.turn[ia];
+            const double rsn = ROT ? A.rot.sn[ia] : 0.0, rcs = ROT ? A.rot.cs[ia] : 1.0;
+
+            // prepare_chip! (src/correlate.jl:423-453): FP64 mean, then the mean-removed Float32
+            // copy, its FP64 sum of squares, and the FP64 sum of the rounded copy. The values are
+            // first staged as Float32 (exact for every type).
+            // The first angle loads the chip, with _any_valid over it (src/track.jl:416-421); the
+            // rotation search keeps it and turns it from shared memory.
+            double st[1] = {0.0};
+            int any = 0;
+            if (ia == 0) {
+                float* dst = ROT ? s_raw : s_chip;
+                for (int a = lane; a < ch; a += 32)
+                    for (int b0 = warp; b0 < cw; b0 += 4 * nwarps) {
+                        float v[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const int64_t r = chip_r + a, c = chip_c + min(b0 + u * nwarps, cw - 1);
+                            any |= pixel_at(A.valid, A.nrows, A.ncols, r, c);
+                            v[u] = static_cast<float>(pixel_at(sec, A.nrows, A.ncols, r, c));
+                        }
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            if (b0 + u * nwarps < cw) {
+                                dst[(b0 + u * nwarps) * A.CHP + a] = v[u];
+                                if (!ROT) st[0] = __dadd_rn(st[0], static_cast<double>(v[u]));
+                            }
+                    }
+            }
+            if (ia == 0) {
+                if (!__syncthreads_or(any)) {
+                    skip = true;
+                    break;
+                }
+                if (tid == 0) A.out.searched[k] = 1;
+            }
+            if constexpr (ROT) {
+                for (int b = warp; b < cw; b += nwarps)
+                    for (int a = lane; a < ch; a += 32) {
+                        const float v = turn ? rotated_at(s_raw, A.CHP, ch, cw, a, b, rsn, rcs)
+                                             : s_raw[b * A.CHP + a];
+                        s_chip[b * A.CHP + a] = v;
+                        st[0] = __dadd_rn(st[0], static_cast<double>(v));
+                    }
+            }
+            block_sum_f64<1>(st, s_red);
+            TC_PHASE(0)
+            const double mean = __ddiv_rn(st[0], nn);
+            double acc2[2] = {0.0, 0.0};
+            for (int b = warp; b < cw; b += nwarps)
+                for (int a = lane; a < chp; a += 32) {
+                    float df = 0.0f;
+                    if (a < ch) {
+                        const double d = __dsub_rn(static_cast<double>(s_chip[b * A.CHP + a]), mean);
+                        df = __double2float_rn(d);
+                        acc2[0] = __dadd_rn(acc2[0], __dmul_rn(d, d));
+                        acc2[1] = __dadd_rn(acc2[1], static_cast<double>(df));
+                    }
+                    s_chip[b * A.CHP + a] = df;
+                }
+            block_sum_f64<2>(acc2, s_red);
+            const double sq = acc2[0], sumd = acc2[1];
+            if (!(sq > __dmul_rn(__dmul_rn(DBL_EPSILON, static_cast<double>(ch)),
+                                 static_cast<double>(cw))))
+                continue;  // degenerate chip: no surface at this angle (src/track.jl:286, 326)
+            const double cnorm = __dsqrt_rn(sq);
+            TC_PHASE(1)
+            // Centring constant of the window: a Float32 value, so that W - c rounds once (the
+            // difference is exact for integer types).
+            const float cs = Tr::integer ? static_cast<float>(rint(mean)) : __double2float_rn(mean);
+            const double cshift = static_cast<double>(cs);
+
+            // The window of an integer image is staged for the first angle; another angle's shift is
+            // then added to it (exactly).
+            const bool restage = !Tr::integer || !staged;
+            if (!restage && cs != staged_cs) {
+                const int wrows = nr + ch - 1;
+                const float d = staged_cs - cs;
+                for (int x = warp; x < XW; x += nwarps) {
+                    float2* col = s_win + ((x & 1) * XH + (x >> 1)) * A.WS;
+                    const float dn = x + 1 < XW ? d : 0.0f;
+#pragma unroll 4
+                    for (int r = lane; r < wrows; r += 32) {
+                        const float2 w = col[r];
+                        col[r] = make_float2(w.x + d, w.y + dn);
+                    }
+                }
+            }
+            staged = true;
+            staged_cs = cs;
+            // The window, shifted, zero-padded outside the image before the shift and below its last
+            // row after it: a warp takes a run of columns, lanes the rows, each lane keeping the
+            // column before.
+            if (restage) {
+                const int wrows = nr + ch - 1, srows = ngrp * kMI + chp;
+                const int run = (XW + nwarps - 1) / nwarps;
+                const int x0 = warp * run, x1 = min(x0 + run, XW);
+                // Three row chunks of twelve columns in flight.
+                for (int rb = 0; rb < srows && x0 < x1; rb += 96) {
+                    const T* row[3];
+                    bool rin[3], live[3];
+                    float prev[3];
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) {
+                        const int r = rb + 32 * q + lane;
+                        const int64_t ir = win_r + r;
+                        live[q] = r < wrows;
+                        rin[q] = live[q] && ir >= 0 && ir < A.nrows;
+                        row[q] = ref + (rin[q] ? ir : 0);
+                    }
+                    // Column x of row chunk q, zero outside the image, before the shift; from an
+                    // address that is always valid.
+                    auto load = [&](int x, int q) {
+                        const int64_t c = win_c + x;
+                        const bool in = c >= 0 && c < A.ncols;
+                        const T v = row[q][(in ? c : 0) * A.nrows];
+                        return in && rin[q] ? static_cast<float>(v) : 0.0f;
+                    };
+                    auto shifted = [&](float v, int x, int q) {
+                        return live[q] && x < XW ? __fsub_rn(v, cs) : 0.0f;
+                    };
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) prev[q] = load(x0, q);
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) prev[q] = shifted(prev[q], x0, q);
+                    for (int x = x0; x < x1; x += 12) {
+                        float v[3][12];
+#pragma unroll
+                        for (int u = 0; u < 12; ++u)
+#pragma unroll
+                            for (int q = 0; q < 3; ++q) v[q][u] = load(x + u + 1, q);
+#pragma unroll
+                        for (int u = 0; u < 12; ++u) {
+                            const int xx = x + u;
+                            float2* dst = s_win + ((xx & 1) * XH + (xx >> 1)) * A.WS + rb + lane;
+#pragma unroll
+                            for (int q = 0; q < 3; ++q) {
+                                const float next = shifted(v[q][u], xx + 1, q);
+                                if (xx < x1 && rb + 32 * q + lane < srows) dst[32 * q] = make_float2(prev[q], next);
+                                prev[q] = next;
+                            }
+                        }
+                    }
+                }
+            }
+            __syncthreads();
+            TC_PHASE(2)
+
+            // Box sums of W and W^2 (integral_both!, boxsum, src/integral.jl:141-170, 244-247) in
+            // FP64 from the image values (the staged ones plus the shift: exact for integer types
+            // and zero padding) and each value's variance term max(s2 - s1 s1 / n, 0) (NCC: max(s2,
+            // 0)). A thread slides a column's sums of ch rows down one of `nseg` segments of the
+            // surface rows; A.TI rows of each segment at a time go to shared memory, where a task
+            // sums cw columns for five neighbouring values. The counts of non-zero values keep
+            // windows of zeros at exactly zero, which sliding FP64 sums would miss by a rounding.
+            if (!have_var) {
+                const int nseg = max(1, min(8, kCorrThreads / XW));
+                const int seglen = (nr + nseg - 1) / nseg;
+                const int seg = tid / XW, x = tid - seg * XW;
+                const bool sums = seg < nseg;
+                const int i0 = seg * seglen, i1 = min(i0 + seglen, nr);
+                const float2* col = s_win + ((x & 1) * XH + (x >> 1)) * A.WS;
+                // An image value from its staged one; integers by way of 1.5 x 2^23, whose last bits
+                // hold them.
+                auto value = [&](float v) -> BS {
+                    if constexpr (Tr::integer) {
+                        return static_cast<BS>(__float_as_int(__fadd_rn(__fadd_rn(v, cs), 12582912.0f)) - 0x4B400000);
+                    } else {
+                        return __dadd_rn(static_cast<double>(v), cshift);
+                    }
+                };
+                BS h1 = 0, h2 = 0;
+                int nz = 1;  // non-zero values (Float32: the others' sums are exact)
+                if (sums && i0 < i1) {
+                    BS a1[4] = {0, 0, 0, 0}, a2[4] = {0, 0, 0, 0};
+                    if (!Tr::integer) nz = 0;
+                    int a = 0;
+#pragma unroll 2
+                    for (; a + 4 <= ch; a += 4)
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const BS w = value(col[i0 + a + u].x);
+                            a1[u] += w;
+                            a2[u] += w * w;
+                            if (!Tr::integer) nz += w != BS(0);
+                        }
+                    for (; a < ch; ++a) {
+                        const BS w = value(col[i0 + a].x);
+                        a1[0] += w;
+                        a2[0] += w * w;
+                        if (!Tr::integer) nz += w != BS(0);
+                    }
+                    h1 = (a1[0] + a1[1]) + (a1[2] + a1[3]);
+                    h2 = (a2[0] + a2[1]) + (a2[2] + a2[3]);
+                }
+                const bool p2 = ((ch * cw) & (ch * cw - 1)) == 0;
+                const double inv = 1.0 / nn;
+                const int slots = nseg * A.TI, jtasks = slots * ((nc + 4) / 5);
+                for (int t0 = 0; t0 < seglen; t0 += A.TI) {
+                    // Four rows at a time, their values loaded before the sums are stored (the stores
+                    // may alias the window as far as the compiler knows).
+                    for (int t = 0; sums && t < A.TI; t += 4) {
+                        const int i = i0 + t0 + t;
+                        if (i >= i1) break;
+                        float fo[4], fn[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            fo[u] = col[min(i + u, i1 - 1)].x;
+                            fn[u] = col[min(i + u, i1 - 1) + ch].x;
+                        }
+                        BS e1[4], e2[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            e1[u] = nz ? h1 : BS(0);
+                            e2[u] = nz ? h2 : BS(0);
+                            const BS wo = value(fo[u]), wn = value(fn[u]);
+                            h1 += wn - wo;
+                            h2 += wn * wn - wo * wo;
+                            if (!Tr::integer) nz += (wn != BS(0)) - (wo != BS(0));
+                        }
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            if (t + u < A.TI && i + u < i1) {
+                                s_v1[(seg * A.TI + t + u) * XW + x] = e1[u];
+                                s_v2[(seg * A.TI + t + u) * XW + x] = e2[u];
+                            }
+                    }
+                    __syncthreads();
+                    for (int task = tid; task < jtasks; task += kCorrThreads) {
+                        const int jg = task / slots, sl = task - jg * slots;
+                        const int sg = sl / A.TI, t = t0 + sl - sg * A.TI;
+                        const int i = sg * seglen + t, j0 = 5 * jg;
+                        if (t >= seglen || i >= nr) continue;
+                        const BS* v1 = s_v1 + sl * XW + j0;
+                        const BS* v2 = s_v2 + sl * XW + j0;
+                        BS a1[4] = {0, 0, 0, 0}, a2[4] = {0, 0, 0, 0};
+                        int n = Tr::integer ? 1 : 0, b = 0;
+#pragma unroll 2
+                        for (; b + 4 <= cw; b += 4)
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) {
+                                const BS w2 = v2[b + u];
+                                a1[u] += v1[b + u];
+                                a2[u] += w2;
+                                if (!Tr::integer) n += w2 != BS(0);
+                            }
+                        for (; b < cw; ++b) {
+                            a1[0] += v1[b];
+                            a2[0] += v2[b];
+                            if (!Tr::integer) n += v2[b] != BS(0);
+                        }
+                        BS g1[5], g2[5];
+                        int ng[5];
+                        g1[0] = (a1[0] + a1[1]) + (a1[2] + a1[3]);
+                        g2[0] = (a2[0] + a2[1]) + (a2[2] + a2[3]);
+                        ng[0] = n;
+                        const int last = nc - 1 - j0;  // columns past the surface repeat its last one
+#pragma unroll
+                        for (int m = 1; m < 5; ++m) {
+                            const int o = max(min(m, last) - 1, 0);
+                            const BS o2 = v2[o], n2 = v2[o + cw];
+                            g1[m] = g1[m - 1] + (v1[o + cw] - v1[o]);
+                            g2[m] = g2[m - 1] + (n2 - o2);
+                            ng[m] = ng[m - 1];
+                            if (!Tr::integer) ng[m] += (n2 != BS(0)) - (o2 != BS(0));
+                        }
+#pragma unroll
+                        for (int m = 0; m < 5; ++m) {
+                            const double s1 = static_cast<double>(g1[m]), s2 = static_cast<double>(g2[m]);
+                            double wvar = s2;
+                            if (A.measure != AR_NCC) {
+                                const double q = __dmul_rn(s1, s1);
+                                wvar = __dsub_rn(s2, p2 ? __dmul_rn(q, inv) : __ddiv_rn(q, nn));
+                            }
+                            if (m <= last) s_wv[(j0 + m) * A.NRS + i] = ng[m] && wvar > 0.0 ? wvar : 0.0;
+                        }
+                    }
+                    __syncthreads();
+                }
+                have_var = Tr::integer;  // Float32 image values carry the shift's rounding
+            }
+
+            TC_PHASE(3)
+            // Numerator: kMI rows of two columns per thread over its part of the chip columns.
+            double acc64[2 * kMI];
+#pragma unroll
+            for (int v = 0; v < 2 * kMI; ++v) acc64[v] = 0.0;
+            if (active) {
+                const int ncg = cw >> 1;  // groups of two chip columns
+                const int ge = ncg * (part + 1) / split;
+                for (int gc = ncg * part / split; gc < ge; ++gc) {
+                    float2 acc[kMI];
+#pragma unroll
+                    for (int m = 0; m < kMI; ++m) acc[m] = make_float2(0.0f, 0.0f);
+#pragma unroll 1
+                    for (int bb = 0; bb < 2; ++bb) {
+                        const float2* wc = s_win + (bb * XH + p + gc) * A.WS + il;
+                        const float4* cc = reinterpret_cast<const float4*>(s_chip + (2 * gc + bb) * A.CHP);
+                        float2 w[kMI + 8];
+#pragma unroll
+                        for (int m = 0; m < kMI; ++m) w[m] = wc[m];
+                        wc += kMI;
+                        // The chip values of the next step are loaded a step ahead (past the last one
+                        // they are the next column's, or the window's, and unused).
+                        float4 c0 = cc[0], c1 = cc[1];
+#pragma unroll 2
+                        for (int a0 = 0; a0 < chp; a0 += 8) {
+#pragma unroll
+                            for (int m = 0; m < 8; ++m) w[kMI + m] = wc[a0 + m];
+                            const float c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+                            c0 = cc[(a0 >> 2) + 2];
+                            c1 = cc[(a0 >> 2) + 3];
+#pragma unroll
+                            for (int a = 0; a < 8; ++a)
+#pragma unroll
+                                for (int m = 0; m < kMI; ++m)
+                                    acc[m] = __ffma2_rn(make_float2(c[a], c[a]), w[m + a], acc[m]);
+#pragma unroll
+                            for (int m = 0; m < kMI; ++m) w[m] = w[m + 8];
+                        }
+                    }
+#pragma unroll
+                    for (int m = 0; m < kMI; ++m) {
+                        acc64[2 * m] = __dadd_rn(acc64[2 * m], static_cast<double>(acc[m].x));
+                        acc64[2 * m + 1] = __dadd_rn(acc64[2 * m + 1], static_cast<double>(acc[m].y));
+                    }
+                }
+            }
+            TC_PHASE(4)
+            // The parts' sums: halves until two are left, which then keep half of the rows each.
+            for (int h = split >> 1; h > 1; h >>= 1) {
+                __syncthreads();
+                if (active && part >= h && part < 2 * h)
+#pragma unroll
+                    for (int v = 0; v < 2 * kMI; ++v) s_ex[v * (kCorrThreads / 2) + tid - h * items] = acc64[v];
+                __syncthreads();
+                if (part < h)
+#pragma unroll
+                    for (int v = 0; v < 2 * kMI; ++v)
+                        acc64[v] = __dadd_rn(acc64[v], s_ex[v * (kCorrThreads / 2) + tid]);
+            }
+            if (split > 1) {
+                __syncthreads();
+                if (part < 2)
+#pragma unroll
+                    for (int v = 0; v < 2 * kMI; ++v)
+                        if ((v < kMI) != (part == 0)) s_ex[v * (kCorrThreads / 2) + it] = acc64[v];
+                __syncthreads();
+                if (part < 2)
+#pragma unroll
+                    for (int v = 0; v < 2 * kMI; ++v)
+                        if ((v < kMI) == (part == 0)) acc64[v] = __dadd_rn(acc64[v], s_ex[v * (kCorrThreads / 2) + it]);
+            }
+            TC_PHASE(5)
+            // Value v of this thread is surface row il + v / 2, column 2 p + v % 2.
+            auto mine = [&](int v) {
+                return (split == 1 ? part == 0 : part < 2 && (v < kMI) == (part == 0)) && il + (v >> 1) < nr;
+            };
+            const double add = __dmul_rn(cshift, sumd);
+#pragma unroll
+            for (int v = 0; v < 2 * kMI; ++v) acc64[v] = __dadd_rn(acc64[v], add);
+
+            // Float32 estimates num rsqrt(wvar), within 8 x 2^-24 of cnorm times the value they stand
+            // for; 0 where there is no variance (the value is 0). `odd`: a magnitude that Float32
+            // cannot be trusted with, or a NaN: then every value is evaluated exactly. The largest
+            // and second largest of each thread, then of each warp.
+            auto estimate = [&](int v, bool& bad) {
+                const double wvar = s_wv[(2 * p + (v & 1)) * A.NRS + il + (v >> 1)];
+                const float n = __double2float_rn(acc64[v]), w = __double2float_rn(wvar);
+                if (!(wvar > 0.0)) return 0.0f;
+                bad |= !(w > 1e-30f && w < 1e30f && fabsf(n) < 1e30f);
+                return __fmul_rn(n, rsqrtf(w));
+            };
+            bool odd = false;
+            float own = -INFINITY, own2 = -INFINITY;
+            int at = 0;
+#pragma unroll
+            for (int v = 0; v < 2 * kMI; ++v)
+                if (mine(v)) {
+                    const float e = estimate(v, odd);
+                    own2 = fmaxf(own2, fminf(own, e));
+                    at = e > own ? v : at;
+                    own = fmaxf(own, e);
+                }
+            {
+                const float top = warp_max(own);
+                const unsigned who = __ballot_sync(kFull, own == top && own > -INFINITY);
+                const int first = who ? __ffs(who) - 1 : 0;
+                const float sec_ = warp_max(odd ? INFINITY : lane == first ? own2 : own);
+                if (lane == first) {
+                    s_top[warp] = top;
+                    s_sec[warp] = sec_;
+                    s_at[warp] = ((il + (at >> 1)) << 16) | (2 * p + (at & 1));
+                }
+            }
+            __syncthreads();  // also: s_ex is read
+            TC_PHASE(6)
+            const float wt = lane < nwarps ? s_top[lane] : -INFINITY;
+            const float M = warp_max(wt);
+            const float cut = M - 1.9073486e-06f * fabsf(M);  // 32 x 2^-24
+            const int mw = __ffs(__ballot_sync(kFull, wt == M)) - 1;
+            const bool unique =
+                fabsf(M) > 1e-30f && fabsf(M) < 1e37f &&
+                !__any_sync(kFull, lane < nwarps && (!(s_sec[lane & 7] < cut) || (lane != mw && !(wt < cut))));
+            int pi = 0, pj = 0;
+            bool any_peak = true;
+            if (unique && !A.surf_out) {
+                // Every other value is below this one: it is the strict (so the first) maximum.
+                pi = s_at[mw] >> 16;
+                pj = s_at[mw] & 0xFFFF;
+            } else {
+                const bool all = __syncthreads_or(odd) || !(fabsf(M) > 1e-30f && fabsf(M) < 1e37f);
+                unsigned long long key = 0ull;
+#pragma unroll
+                for (int v = 0; v < 2 * kMI; ++v)
+                    if (mine(v) && (all || A.surf_out || !(estimate(v, odd) < cut))) {
+                        const int i = il + (v >> 1), j = 2 * p + (v & 1);
+                        const float x = fp_exact(acc64[v], s_wv[j * A.NRS + i], cnorm);
+                        const unsigned long long kk = argmax_key(x, static_cast<unsigned>(i * nc + j));
+                        key = kk > key ? kk : key;
+                        if (A.surf_out) A.surf_out[k * static_cast<int64_t>(A.NRS) * A.NCM + i + j * nr] = x;
+                    }
+                key = block_max_u64(key, reinterpret_cast<unsigned long long*>(s_red));
+                unsigned rm = 0;
+                float pv = 0.0f;
+                any_peak = key != 0ull;
+                if (key_decode(key, &rm, &pv)) {
+                    pi = static_cast<int>(rm / nc);
+                    pj = static_cast<int>(rm % nc);
+                }
+            }
+            TC_PHASE(7)
+            if (A.flops && tid == 0)
+                atomicAdd(A.flops, 2ull * static_cast<unsigned long long>(ch) * cw * nr * nc);
+
+            // The peak's value or the 5x5 patch's (src/peak.jl:473-482), exactly, a thread each; with
+            // the rotation search kept if the angle's maximum (src/track.jl:327-328) is the largest.
+            const int qi = single ? pi : min(max(pi - 2, 0), max(nr - 5, 0));
+            const int qj = single ? pj : min(max(pj - 2, 0), max(nc - 5, 0));
+            const unsigned span = single ? 1u : 5u;
+            if (qi < il + kMI && qi + static_cast<int>(span) > il && qj <= 2 * p + 1 &&
+                qj + static_cast<int>(span) > 2 * p) {
+#pragma unroll
+                for (int v = 0; v < 2 * kMI; ++v) {
+                    const int i = il + (v >> 1), j = 2 * p + (v & 1);
+                    const unsigned a = static_cast<unsigned>(i - qi), c = static_cast<unsigned>(j - qj);
+                    if (a < span && c < span && mine(v)) {
+                        s_pn[c * 5 + a] = acc64[v];
+                        s_pw[c * 5 + a] = s_wv[j * A.NRS + i];
+                    }
+                }
+            }
+            __syncthreads();
+            const int npatch = single ? 1 : 25;
+            if constexpr (!ROT) {
+                found = true;
+                pi0 = qi;
+                pj0 = qj;
+                if (tid < npatch) s_best[tid] = fp_exact(s_pn[tid], s_pw[tid], cnorm);
+            } else {
+                if (tid < npatch) s_pp[tid] = fp_exact(s_pn[tid], s_pw[tid], cnorm);
+                __syncthreads();
+                const float pk = any_peak ? s_pp[(pj - qj) * 5 + (pi - qi)] : NAN;
+                if (pk > bestpk) {
+                    bestpk = pk;
+                    found = true;
+                    pi0 = qi;
+                    pj0 = qj;
+                    if (tid < npatch) s_best[tid] = s_pp[tid];
+                }
+            }
+            TC_PHASE(8)
+        }
+        if (skip || !found) continue;  // every angle degenerate: searched, no measurement
+        // Warp 0 has the values (it computed them).
+        if (warp == 0) {
+            if (single) {
+                // peak_offset (src/peak.jl:102-106) and the output write (src/track.jl:293-295).
+                if (lane == 0) {
+                    A.out.dx[k] = __double2float_rn(__dadd_rn(static_cast<double>(pj0 - static_cast<int>(prx)), dx0));
+                    A.out.dy[k] = __double2float_rn(__dadd_rn(static_cast<double>(pi0 - static_cast<int>(pry)), dy0));
+                    A.out.corr[k] = s_best[0];
+                }
+            } else {
+                int slot = 0;
+                if (lane == 0) slot = atomicAdd(A.sub_count, 1);
+                slot = __shfl_sync(kFull, slot, 0);
+                if (lane < 25) A.sub_patch[static_cast<int64_t>(slot) * 25 + lane] = s_best[lane];
+                if (lane == 0) {
+                    A.sub_point[slot] = k;
+                    A.sub_origin[2 * slot] = pi0;
+                    A.sub_origin[2 * slot + 1] = pj0;
+                }
+            }
+        }
+        TC_PHASE(9)
+        TC_PHASE_POINT
+    }
+    TC_PHASE_FLUSH
+}
+
 // ----------------------------------------------------------------------------------------------
 // Tensor-core correlation for UInt8 imagery (tcgen05.mma kind::i8, exact 32-bit accumulation).
 //
@@ -941,32 +1627,6 @@ __device__ __forceinline__ void staged_chip_stats(const uint8_t* s_P, int PC, in
     block_sum_f64<1, MAIN>(acc2, s_red);
     *sq = acc2[0];
 }
-
-// Optional phase timer (compiled in with -DAR_TC_PHASES, for profiling builds only): thread 0
-// of each CTA accumulates clock64() cycles between the marks below, per phase, and adds them to
-// g_tc_phase at exit; entry 15 counts the points that reached the output phase.
-#ifdef AR_TC_PHASES
-__device__ unsigned long long g_tc_phase[16];
-#define TC_PHASE_INIT unsigned long long tcp_t = clock64(), tcp_acc[12] = {}, tcp_n = 0;
-#define TC_PHASE(n)                              \
-    if (tid == 0) {                              \
-        const unsigned long long t_ = clock64(); \
-        tcp_acc[n] += t_ - tcp_t;                \
-        tcp_t = t_;                              \
-    }
-#define TC_PHASE_POINT \
-    if (tid == 0) ++tcp_n;
-#define TC_PHASE_FLUSH                                                           \
-    if (tid == 0) {                                                              \
-        for (int n_ = 0; n_ < 12; ++n_) atomicAdd(&g_tc_phase[n_], tcp_acc[n_]); \
-        atomicAdd(&g_tc_phase[15], tcp_n);                                       \
-    }
-#else
-#define TC_PHASE_INIT
-#define TC_PHASE(n)
-#define TC_PHASE_POINT
-#define TC_PHASE_FLUSH
-#endif
 
 // REG: every surface of the pass has at most 64 rows and 64 columns (M = 64), so one 16x256b
 // read per warp covers it and each thread keeps its 16 numerators and upper bounds in
@@ -4059,6 +4719,54 @@ bool plan_corr(const PassGeometry& g, size_t ph_bytes, size_t smem_cap, CorrPlan
     return false;
 }
 
+// Plan of k_corr_fp; false when the surface exceeds one tile (a row group of a column pair per
+// thread), the window one column per thread, or shared memory.
+bool plan_corr_fp(const PassGeometry& g, size_t smem_cap, bool rot, bool integer, CorrPlan* P) {
+    if (g.max_ch > 1024 || g.max_cw > 1024 || g.max_nr > 512 || g.max_nc > 512) return false;
+    const int ch = static_cast<int>(g.max_ch), cw = static_cast<int>(g.max_cw);
+    const int nr = static_cast<int>(g.max_nr), nc = static_cast<int>(g.max_nc);
+    if (ch < 2 || cw < 2 || nr < 2 || nc < 2) return false;
+    if (ch * cw > 66000) return false;  // UInt8 sums of squares stay below 2^32
+    const int ngrp = (nr + kMI - 1) / kMI;
+    if (ngrp * (nc / 2) > kCorrThreads || cw + nc - 1 > kCorrThreads) return false;
+    P->CHP = round_up(ch, kUA);
+    P->CWM = cw;
+    P->NRS = nr | 1;
+    P->NCM = nc;
+    P->BC = cw;
+    P->TJ = P->PHS = 0;
+    P->WS = (ngrp * kMI + P->CHP) | 1;  // pairs; odd
+    auto a16 = [](size_t v) { return (v + 15) & ~size_t(15); };
+    size_t off = a16(static_cast<size_t>(cw) * P->CHP * 4);
+    P->off_win = static_cast<unsigned>(off);
+    // Every column's run of rows is read to its end by the products' loads.
+    const size_t win = static_cast<size_t>(2 * ((cw + nc) / 2)) * P->WS * 8 + 128;
+    // The partial sums of split products (20 FP64 values of half of the threads) take the window's
+    // place; with the rotation search of an integer image, whose window stays, the column sums',
+    // which are done by then.
+    const size_t ex = static_cast<size_t>(2 * kMI) * (kCorrThreads / 2) * 8;
+    const bool keep = rot && integer;
+    P->off_surf2 = static_cast<unsigned>(off);
+    off += a16(keep ? win : std::max(win, ex));
+    P->off_ph1 = static_cast<unsigned>(off);
+    if (keep) P->off_surf2 = static_cast<unsigned>(off);
+    // Rows of each segment's column sums: eight where two CTAs per SM (112 KB each) still fit, else
+    // four.
+    const size_t raw = rot ? a16(static_cast<size_t>(cw) * P->CHP * 4) : 0;
+    const size_t rest = raw + a16(static_cast<size_t>(nc) * P->NRS * 8) + 3 * 32 * 8;
+    const size_t row = 2 * static_cast<size_t>(kCorrThreads) * 8;
+    P->TI = off + std::max(8 * row, keep ? ex : 0) + rest <= 111 * 1024 ? 8 : 4;
+    off += std::max(P->TI * row, keep ? ex : 0);
+    P->off_ph2 = static_cast<unsigned>(off);
+    off += a16(static_cast<size_t>(nc) * P->NRS * 8);
+    P->off_surf = static_cast<unsigned>(off);
+    off += raw;
+    P->off_red = static_cast<unsigned>(off);
+    off += 3 * 32 * 8;
+    P->smem = off;
+    return off <= smem_cap;
+}
+
 int ilog2_exact(int up) {
     int L = 0;
     while ((1 << L) < up) ++L;
@@ -4427,9 +5135,16 @@ bool plan_corr_tc(const PassGeometry& g, size_t smem_cap, TcPlan* P) {
 }
 
 template <typename T>
-cudaError_t launch_corr_t(const CorrArgs& A, const CorrPlan& P, int grid, cudaStream_t stream) {
+cudaError_t launch_corr_t(const CorrArgs& A, const CorrPlan& P, int grid, cudaStream_t stream, bool fp) {
     if (P.smem > static_cast<size_t>(kDynSmemCap)) return cudaErrorInvalidValue;
     auto kern = A.rot.count > 0 ? k_corr<T, true> : k_corr<T, false>;
+    if (fp) {
+        if constexpr (Traits<T>::raw) {
+            kern = k_corr_fp<T, true>;  // the integer numerator stays with k_corr
+        } else {
+            kern = A.rot.count > 0 ? k_corr_fp<T, true> : k_corr_fp<T, false>;
+        }
+    }
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          kDynSmemCap);
     if (e != cudaSuccess) return e;
@@ -4726,7 +5441,11 @@ cudaError_t launch_track_impl(int dtype, const void* ref, const void* sec, const
     const bool rotating = rot && rot->count > 0;
     const size_t ph_bytes = dtype == AR_U8 && !rotating ? 4 : 8;
     CorrPlan P{};
-    if (!plan_corr(geom, ph_bytes, 220 * 1024, &P, rotating)) {
+    // One-tile surfaces with an FP32 numerator take k_corr_fp: turned chips (but not with a
+    // diagnostic surface, which k_corr keeps across angles) and the types other than UInt8.
+    const bool fp = (rotating ? !surf_out : dtype != AR_U8) && 
+                    plan_corr_fp(geom, 220 * 1024, rotating, dtype != AR_F32, &P);
+    if (!fp && !plan_corr(geom, ph_bytes, 220 * 1024, &P, rotating)) {
         if (err) *err = rotating ? "chip and search geometry too large for shared memory with "
                                    "the rotation search"
                                  : "chip and search geometry too large for shared memory";
@@ -4869,10 +5588,10 @@ cudaError_t launch_track_impl(int dtype, const void* ref, const void* sec, const
         const int64_t want = static_cast<int64_t>(num_sms) * per_sm * 8;
         const int grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(pts_.n, want)));
         switch (dtype) {
-            case AR_U8: return launch_corr_t<uint8_t>(A2, P, grid, stream);
-            case AR_U16: return launch_corr_t<uint16_t>(A2, P, grid, stream);
-            case AR_I16: return launch_corr_t<int16_t>(A2, P, grid, stream);
-            case AR_F32: return launch_corr_t<float>(A2, P, grid, stream);
+            case AR_U8: return launch_corr_t<uint8_t>(A2, P, grid, stream, fp);
+            case AR_U16: return launch_corr_t<uint16_t>(A2, P, grid, stream, fp);
+            case AR_I16: return launch_corr_t<int16_t>(A2, P, grid, stream, fp);
+            case AR_F32: return launch_corr_t<float>(A2, P, grid, stream, fp);
             default: return cudaErrorInvalidValue;
         }
     };
