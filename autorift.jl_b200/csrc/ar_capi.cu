@@ -14,6 +14,7 @@
 #include <mutex>
 #include <string>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "ar_internal.cuh"
@@ -313,29 +314,86 @@ cudaError_t ensure_dbuf(ar_ctx* c, size_t bytes) {
 }
 
 // Per-image masks (given ones normalised to 0/1, missing ones from finiteness, the ImagePair
-// default of src/preprocess.jl:74-79) and their intersection, valid(pair).
+// default of src/preprocess.jl:74-79) and their intersection, valid(pair). A thread takes kMaskRun
+// consecutive pixels, as 16-byte words where the arrays are aligned (a byte a thread ran at a
+// quarter of the memory bandwidth: 126 us for a 6001 x 5003 pair; 24 now).
+constexpr int kMaskRun = 16;
+
+struct alignas(16) MaskWord {
+    uint8_t x[kMaskRun];
+};
+
+__device__ __forceinline__ bool mask_aligned(const uint8_t* a, const uint8_t* b, const uint8_t* c) {
+    return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) |
+             reinterpret_cast<uintptr_t>(c)) & 15u) == 0;
+}
+
+// `out` = fn(index) for the run that starts at pixel i of n.
+template <typename Fn>
+__device__ __forceinline__ void mask_store(uint8_t* out, int64_t i, int64_t n, bool vec, Fn fn) {
+    MaskWord w;
+#pragma unroll
+    for (int e = 0; e < kMaskRun; ++e) w.x[e] = fn(e);
+    if (vec && i + kMaskRun <= n) {
+        *reinterpret_cast<MaskWord*>(out + i) = w;
+    } else {
+        for (int e = 0; e < kMaskRun; ++e)
+            if (i + e < n) out[i + e] = w.x[e];
+    }
+}
+__device__ __forceinline__ MaskWord mask_load(const uint8_t* m, int64_t i, int64_t n, bool vec) {
+    MaskWord w;
+    if (vec && i + kMaskRun <= n) return *reinterpret_cast<const MaskWord*>(m + i);
+#pragma unroll
+    for (int e = 0; e < kMaskRun; ++e) w.x[e] = i + e < n ? m[i + e] : 0;
+    return w;
+}
+
 template <typename T>
 __global__ void k_make_valid(const T* ref, const T* sec, uint8_t* rv, uint8_t* sv, bool have_rv,
                              bool have_sv, uint8_t* out, int64_t n) {
-    const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+    const int64_t i = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) * kMaskRun;
     if (i >= n) return;
-    const bool a = have_rv ? rv[i] != 0 : isfinite(static_cast<double>(ref[i]));
-    const bool b = have_sv ? sv[i] != 0 : isfinite(static_cast<double>(sec[i]));
-    rv[i] = a ? 1 : 0;
-    sv[i] = b ? 1 : 0;
-    out[i] = (a && b) ? 1 : 0;
+    const bool vec = mask_aligned(rv, sv, out);
+    auto side = [&](const T* img, uint8_t* m, bool have) {
+        MaskWord w;
+        if (have) {
+            w = mask_load(m, i, n, vec);
+        } else {
+#pragma unroll
+            for (int e = 0; e < kMaskRun; ++e)
+                w.x[e] = std::is_floating_point<T>::value
+                             ? (i + e < n && isfinite(static_cast<double>(img[i + e])) ? 1 : 0)
+                             : 1;
+        }
+        mask_store(m, i, n, vec, [&](int e) -> uint8_t { return w.x[e] ? 1 : 0; });
+        return w;
+    };
+    const MaskWord a = side(ref, rv, have_rv), b = side(sec, sv, have_sv);
+    mask_store(out, i, n, vec, [&](int e) -> uint8_t { return a.x[e] && b.x[e] ? 1 : 0; });
 }
 
 __global__ void k_and_masks(const uint8_t* a, const uint8_t* b, uint8_t* out, int64_t n) {
-    const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (i < n) out[i] = (a[i] && b[i]) ? 1 : 0;
+    const int64_t i = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) * kMaskRun;
+    if (i >= n) return;
+    const bool vec = mask_aligned(a, b, out);
+    const MaskWord u = mask_load(a, i, n, vec), v = mask_load(b, i, n, vec);
+    mask_store(out, i, n, vec, [&](int e) -> uint8_t { return u.x[e] && v.x[e] ? 1 : 0; });
+}
+
+// Bytes from one of a pair's three masks to the next: whole 256-byte blocks, so that each is aligned.
+int64_t mask_pitch(int64_t n) { return (n + 255) / 256 * 256; }
+
+unsigned mask_blocks(int64_t n, int threads) {
+    const int64_t per = static_cast<int64_t>(threads) * kMaskRun;
+    return static_cast<unsigned>((n + per - 1) / per);
 }
 
 template <typename T>
 cudaError_t launch_make_valid(ar_pair* p, bool have_rv, bool have_sv, cudaStream_t s) {
     const int threads = 256;
     const int64_t n = p->nrows * p->ncols;
-    k_make_valid<T><<<static_cast<unsigned>((n + threads - 1) / threads), threads, 0, s>>>(
+    k_make_valid<T><<<mask_blocks(n, threads), threads, 0, s>>>(
         static_cast<const T*>(p->ref), static_cast<const T*>(p->sec), p->ref_valid, p->sec_valid,
         have_rv, have_sv, p->valid, n);
     return cudaGetLastError();
@@ -485,10 +543,10 @@ int ar_pair_upload(ar_ctx* c, const void* ref, const void* sec, const uint8_t* r
     p->ncols = ncols;
     cudaError_t e = dalloc(c, &p->ref, n * es);
     if (e == cudaSuccess) e = dalloc(c, &p->sec, n * es);
-    if (e == cudaSuccess) e = dalloc(c, &p->valid, 3 * n);
+    if (e == cudaSuccess) e = dalloc(c, &p->valid, 3 * mask_pitch(n));
     if (e == cudaSuccess) {
-        p->ref_valid = p->valid + n;
-        p->sec_valid = p->valid + 2 * n;
+        p->ref_valid = p->valid + mask_pitch(n);
+        p->sec_valid = p->valid + 2 * mask_pitch(n);
     }
     if (e == cudaSuccess) e = stage_h2d(c, p->ref, ref, n * es);
     if (e == cudaSuccess) e = stage_h2d(c, p->sec, sec, n * es);
@@ -821,10 +879,10 @@ int ar_prepare(ar_ctx* c, const ar_pair* raw, const ar_prepare_opts* opts, ar_pa
     if (c->scratch.done) cudaStreamWaitEvent(c->stream, c->scratch.done, 0);
     cudaError_t e = dalloc(c, &p->ref, n * oes);
     if (e == cudaSuccess) e = dalloc(c, &p->sec, n * oes);
-    if (e == cudaSuccess) e = dalloc(c, &p->valid, 3 * n);
+    if (e == cudaSuccess) e = dalloc(c, &p->valid, 3 * mask_pitch(n));
     if (e == cudaSuccess) {
-        p->ref_valid = p->valid + n;
-        p->sec_valid = p->valid + 2 * n;
+        p->ref_valid = p->valid + mask_pitch(n);
+        p->sec_valid = p->valid + 2 * mask_pitch(n);
     }
     const bool need_f = opts->preprocess != AR_PRE_NONE && opts->quantize == AR_QUANT_UINT8;
     const bool need_m = opts->preprocess == AR_PRE_WALLIS;
@@ -854,8 +912,8 @@ int ar_prepare(ar_ctx* c, const ar_pair* raw, const ar_prepare_opts* opts, ar_pa
     }
     if (e == cudaSuccess) {
         const int threads = 256;
-        k_and_masks<<<static_cast<unsigned>((n + threads - 1) / threads), threads, 0, c->stream>>>(
-            p->ref_valid, p->sec_valid, p->valid, n);
+        k_and_masks<<<mask_blocks(n, threads), threads, 0, c->stream>>>(p->ref_valid, p->sec_valid,
+                                                                        p->valid, n);
         e = cudaGetLastError();
     }
     dfree(c, tmp);
