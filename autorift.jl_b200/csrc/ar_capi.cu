@@ -502,8 +502,6 @@ int ar_ctx_destroy(ar_ctx* c) {
         for (auto ev : c->scratch.timer.pool) cudaEventDestroy(ev);
         cudaFree(c->scratch.timer.flops);
         if (c->scratch.done) cudaEventDestroy(c->scratch.done);
-        for (auto ev : c->scratch.tune_ev)
-            if (ev) cudaEventDestroy(ev);
         cudaFree(c->dbuf);
         cudaFree(c->arena);
         if (c->pinned) cudaFreeHost(c->pinned);

@@ -93,18 +93,16 @@ struct TrackScratch {
     // UInt16, Int16 and Float32 passes: 0 direct FP32 on CUDA cores, 1 split-BF16 tensor-core
     // products for chips of 64 px and up, 2 split-BF16 for every chip size (AR_OPT_SPLIT_BF16).
     int split_bf16 = 1;
-    // UInt8 passes of at least kTuneMinPoints points: the tensor-core and CUDA-core kernels
-    // (identical results) are timed once per pass geometry and the fastest kept in `tuned`
-    // (key: chip and surface extents) -- AR_OPT_AUTOTUNE.
+    // UInt8 passes of at least kTuneMinPoints points enter the kernel their geometry runs in
+    // `tuned` (key: chip and surface extents) -- AR_OPT_AUTOTUNE.
     bool autotune = true;
-    // AR_OPT_UINT8_KERNEL: -1 the autotuner (or the fixed rule); 2, 1, 0 run k_corr_tc2,
+    // AR_OPT_UINT8_KERNEL: -1 the rule; 2, 1, 0 run k_corr_tc2,
     // k_corr_tc or the CUDA-core kernel on every UInt8 pass whose plan fits it.
     int uint8_kernel = -1;
     // Multichip passes whose searchable points have both small (up to 64 x 64) and larger
     // surfaces run each group as its own launch (AR_OPT_SHAPE_BINS).
     bool shape_bins = true;
     std::map<uint64_t, int> tuned;
-    cudaEvent_t tune_ev[2] = {nullptr, nullptr};
     // When set, the sub-pixel queue grows from this pool in stream order (no device-wide
     // synchronisation when a context first meets a larger pass).
     cudaMemPool_t pool = nullptr;

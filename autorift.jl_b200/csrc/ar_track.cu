@@ -5349,76 +5349,8 @@ cudaError_t scratch_acquire(TrackScratch& s, cudaStream_t stream) {
 
 long long scratch_allocations() { return g_scratch_allocs.load(); }
 
-// Passes of at least kTuneMinPoints points are tuned: the tensor-core kernels on their first
-// kTuneSample points, the CUDA-core kernel on the first kTuneSampleDirect.
+// Passes of at least this many points enter the context's table of geometries and kernels.
 constexpr int64_t kTuneMinPoints = 8192;
-constexpr int64_t kTuneSample = 32768;
-constexpr int64_t kTuneSampleDirect = 4096;
-
-// Times each candidate kernel (2 k_corr_tc2, 1 k_corr_tc, 0 k_corr) on a sample of the pass --
-// consecutive points from its middle, written to their own output slots, without refinement
-// (the pass itself then writes the same values there) -- each launched twice and the second
-// timed, and returns in `kind` the one with the least time per point (a tie keeps the earlier
-// candidate). The tensor-core kernels' sample is large enough that each CTA takes a run of
-// consecutive points, as in the full pass: both carry box sums from one point of a run to the
-// next, and on a sample of 4096 points (one or two points per CTA) k_corr_tc2 lost that and the
-// tuner could pick k_corr_tc, 25 % slower on the full pass. The sample comes from the middle
-// because a pass's first points (its first grid columns) lie at the image's edge, where more
-// points are skipped or clipped than elsewhere: on a 4096 x 4096 scene the first 32 768 points of
-// the chip-32 / radius-25 pass made k_corr_tc look faster, and on the whole pass it is 29 %
-// slower (12.9 against 10.0 ms). With diagnostic
-// surfaces (`at_start`) the sample is the pass's first points, whose rows they are.
-template <typename Launch>
-cudaError_t autotune_u8(TrackScratch& scratch, cudaStream_t stream, const DevPoints& pts,
-                        const DevOutputs& out, bool at_start, bool fit2, bool fit1, int* kind,
-                        Launch launch) {
-    cudaError_t e = cudaSuccess;
-    for (int i = 0; i < 2 && e == cudaSuccess; ++i)
-        if (!scratch.tune_ev[i]) {
-            e = cudaEventCreate(&scratch.tune_ev[i]);
-            ++g_scratch_allocs;
-        }
-    if (e != cudaSuccess) return e;
-    float best = INFINITY;
-    int chosen = fit2 ? 2 : 1;
-    const int cand[3] = {2, 1, 0};
-    for (int c : cand) {
-        if ((c == 2 && !fit2) || (c == 1 && !fit1)) continue;
-        const int64_t m = std::min<int64_t>(pts.n, c == 0 ? kTuneSampleDirect : kTuneSample);
-        const int64_t off = at_start ? 0 : (pts.n - m) / 2;
-        DevPoints ds = pts;
-        ds.x += off;
-        ds.y += off;
-        ds.rx += off;
-        ds.ry += off;
-        ds.dx0 += off;
-        ds.dy0 += off;
-        ds.csx += off;
-        ds.csy += off;
-        ds.n = m;
-        DevOutputs dout = out;
-        dout.dx += off;
-        dout.dy += off;
-        dout.corr += off;
-        dout.searched += off;
-        e = launch(c, ds, dout);
-        if (e == cudaSuccess) e = cudaEventRecord(scratch.tune_ev[0], stream);
-        if (e == cudaSuccess) e = launch(c, ds, dout);
-        if (e == cudaSuccess) e = cudaEventRecord(scratch.tune_ev[1], stream);
-        if (e == cudaSuccess) e = cudaEventSynchronize(scratch.tune_ev[1]);
-        float ms = 0.0f;
-        if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, scratch.tune_ev[0], scratch.tune_ev[1]);
-        if (e != cudaSuccess) return e;
-        scratch.timer.launches += 2;
-        const float per_point = ms / static_cast<float>(ds.n);
-        if (per_point < best) {
-            best = per_point;
-            chosen = c;
-        }
-    }
-    *kind = chosen;
-    return cudaSuccess;
-}
 
 cudaError_t launch_track_impl(int dtype, const void* ref, const void* sec, const uint8_t* valid,
                               int64_t nrows, int64_t ncols, const DevPoints& pts,
@@ -5673,10 +5605,12 @@ cudaError_t launch_track_impl(int dtype, const void* ref, const void* sec, const
         }
     }
     if (!bf_done) {
-        // UInt8: the three kernels are exact and give identical results, so the one to run is
-        // a matter of speed -- by default the tensor-core kernel whose plan fits (k_corr_tc2
-        // first); for large passes the autotuner times the candidates once per geometry on a
-        // sample of the pass and the context keeps the fastest.
+        // UInt8: the three kernels are exact and give identical results; the tensor-core kernel
+        // whose plan fits runs, k_corr_tc2 before k_corr_tc. Over chips of 4 to 80 px, radii of 2
+        // to 32 and consecutive or scattered points, k_corr_tc2 took 0.37 to 0.85 of k_corr_tc's
+        // time and at most 0.90 of k_corr's (chip 4, radius 2); where only k_corr_tc fits
+        // (chips of 96 and 128 px, surfaces beyond 64 x 64) it took 0.40 of k_corr's at most. On a
+        // pass of radii 4 to 32 the two tie (73 523 points at chip 16: 3.9 ms).
         TcPlan TP2{}, TP1{};
         const bool fit2 = tc_ok && plan_corr_tc2(geom, 220 * 1024, &TP2);
         const bool fit1 = tc_ok && plan_corr_tc(geom, 220 * 1024, &TP1);
@@ -5689,19 +5623,7 @@ cudaError_t launch_track_impl(int dtype, const void* ref, const void* sec, const
                                  (static_cast<uint64_t>(geom.max_cw) << 32) |
                                  (static_cast<uint64_t>(geom.max_nr) << 16) |
                                  static_cast<uint64_t>(geom.max_nc);
-            auto it = scratch.tuned.find(key);
-            if (it != scratch.tuned.end()) {
-                kind = it->second;
-            } else {
-                e = autotune_u8(scratch, stream, pts, out, surf_out != nullptr, fit2, fit1, &kind,
-                                [&](int kk, const DevPoints& ds, const DevOutputs& dout) -> cudaError_t {
-                                    if (kk == 2) return launch_tc(true, TP2, ds, 1, dout, nullptr);
-                                    if (kk == 1) return launch_tc(false, TP1, ds, 1, dout, nullptr);
-                                    return launch_direct(ds, 1, dout, nullptr);
-                                });
-                if (e != cudaSuccess) return e;
-                scratch.tuned[key] = kind;
-            }
+            scratch.tuned[key] = kind;
         }
         if (kind == 2) {
             e = launch_tc(true, TP2, pts, up, out, A.flops);

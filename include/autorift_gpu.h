@@ -310,15 +310,15 @@ int ar_release(ar_ctx* ctx, ar_ticket ticket);
  * FP32) -- 1 for passes whose chips are 64 px and up, 2 for every chip size, 0 never (direct
  * FP32). Surface values then differ from the FP64 ones by up to a few 1e-6 instead of ~1e-7;
  * the box sums and the normalisation stay FP64.
- * AR_OPT_AUTOTUNE (default 1): for UInt8 passes of 8192 points or more, the kernels that give
- * identical results (the two tensor-core kernels whose plans fit and the CUDA-core kernel) are
- * timed once per pass geometry on a sample of the pass, and the context runs the fastest from
- * then on; 0 always takes the first tensor-core kernel that fits.
+ * AR_OPT_AUTOTUNE (default 1): UInt8 passes of 8192 points or more enter the kernel that runs
+ * their geometry in the context's table (ar_ctx_tuned); 0 keeps no table. Of the kernels that
+ * give identical results the first whose plan fits runs either way: k_corr_tc2, k_corr_tc, the
+ * CUDA-core kernel.
  * AR_OPT_SHAPE_BINS (default 1): a multichip pass whose searchable points include both surfaces
  * of at most 64 x 64 and larger ones runs the two groups as separate launches, each planned for
  * its own largest surface (per-point radii); 0 runs every pass as one launch. Results are the
  * same either way.
- * AR_OPT_UINT8_KERNEL (default -1: the autotuner, or the fixed rule above): 2, 1 or 0 runs
+ * AR_OPT_UINT8_KERNEL (default -1: the rule above): 2, 1 or 0 runs
  * every UInt8 pass on k_corr_tc2, k_corr_tc or the CUDA-core kernel where that kernel's plan
  * fits the pass (else the usual choice) -- for benchmarks and profiles; results are identical.
  * AR_OPT_SERVE_SLOTS and AR_OPT_SERVE_MEMORY_MB configure the request loop (see ar_submit);
@@ -366,10 +366,10 @@ int ar_kernel_times(ar_ctx* ctx, double* corr_ms, double* refine_ms, int64_t* tr
                     int64_t* launches, double* corr_flops);
 
 /*
- * The UInt8 correlation kernel the autotuner kept for each pass geometry it has timed in this
- * context (AR_OPT_AUTOTUNE): five int32 per geometry -- largest chip rows, chip columns,
+ * The UInt8 correlation kernel that runs each large pass geometry this context has met
+ * (AR_OPT_AUTOTUNE): five int32 per geometry -- largest chip rows, chip columns,
  * surface rows, surface columns, then the kernel (2: k_corr_tc2, 1: k_corr_tc, 0: k_corr, the
- * CUDA-core direct sum). Writes up to `cap` geometries to `out`; *count = the number tuned.
+ * CUDA-core direct sum). Writes up to `cap` geometries to `out`; *count = the number of them.
  * Diagnostics for benchmarks; no reference counterpart.
  */
 int ar_ctx_tuned(ar_ctx* ctx, int32_t* out, int64_t cap, int64_t* count);
