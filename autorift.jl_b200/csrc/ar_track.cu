@@ -1341,9 +1341,17 @@ __global__ void __launch_bounds__(kCorrThreads, 2) k_corr_fp(const CorrArgs A) {
 // kernel's and every surface value, the peak and the patch are bit-identical to it.
 //
 // Normalising all 2ry x 2rx values in FP64 would cost as much as the products, and only the
-// peak and its 5 x 5 patch are read. So each value is first estimated in FP32 together with a
-// rigorous bound on its distance from the FP32 surface value; only values whose bound reaches
+// peak and its 5 x 5 patch are read. So each value is first estimated in FP32 with a
+// rigorous bound on its distance from the FP32 surface value (a bound a value for surfaces up to
+// 64 x 64, one for all of them beyond); only values whose bound reaches
 // the largest estimate, and the patch, get the reference's exact FP64 normalisation.
+//
+// What bounds the larger surfaces: the products' operand reads (6 KB of shared memory a
+// 128 x 64 x 32 product, 884 KB a point at chip 32, surface 88 x 88, some 7 k cycles), then the
+// latency of every other step at eight warps. So the numerators stay in Tensor Memory, nothing
+// but the box sums is kept for each value, and two CTAs share an SM up to 94 x 94 at chip 32 and
+// 96 x 96 at chip 16: 14 400 points of chip 32, radius 44 took 1.67 ms and take 1.19 ms, 12 000 of chip 16,
+// radius 48 0.93 ms (1.42). One CTA of 512 threads, or four issuing threads, gave nothing.
 
 constexpr int kTcThreads = 256;
 constexpr int kTc2Threads = 320;  // k_corr_tc2: eight main warps, a fetch warp, a patch warp
@@ -1358,16 +1366,15 @@ struct TcArgs {
     DevPoints pts;
     int64_t padx, pady;
     int up, measure;
-    int NB, QM, QS, PS, PC, XS, XT, NRS, NRM, NCM, CHM, CWM;
+    int NB, QM, QS, PS, PC, XS, NRS, NRM, NCM, CHM, CWM;
     int BC;                          // chip columns per chunk of the chip operand (even)
     int MT;                          // MMA M: 64 or 128 surface columns
     int big;                         // 1: box sums before the products, chunks reuse their space
-                                     // 2: the same in stripes of VR surface rows
-    int VR;                          // k_corr_tc, big == 2: surface rows per box-sum stripe
-    unsigned off_E, off_W, off_T, off_P, off_V, off_S1, off_S2, off_num, off_est, off_red;
+    int VR;                          // k_corr_tc: surface rows per box-sum stripe
+    int roots;                       // k_corr_tc: reciprocal roots kept beside the box sums
+    unsigned off_E, off_W, off_P, off_V, off_S1, off_S2, off_R, off_num, off_est, off_red;
     unsigned off_L, off_rawW, off_rawC;  // k_corr_tc2
-    int XV;                          // row stride (words) of the column sums V1, V2 (k_corr_tc2;
-                                     // k_corr_tc with big == 2)
+    int XV;                          // row stride (words) of the column sums V1, V2
     int acc1_col;                    // stride between the accumulators (first column of the
                                      // second one)
     int issuers;                     // k_corr_tc: threads issuing the products, 2 or 4
@@ -1438,44 +1445,7 @@ __device__ __forceinline__ float tc_estimate(uint32_t D, uint32_t S1, uint32_t S
     return est;
 }
 
-// tc_estimate for two values at once on packed FP32 pairs: every operation rounds each lane as
-// the scalar form does, so the estimates and bounds are the scalar ones bit for bit.
 __device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
-__device__ __forceinline__ float2 tc_estimate2(uint32_t D0, uint32_t D1, uint32_t S10,
-                                               uint32_t S11, uint32_t S20, uint32_t S21,
-                                               float nnf, float csum, float k, float k7,
-                                               int measure, float2* bound) {
-    const float2 d = make_float2(__uint2float_rn(D0), __uint2float_rn(D1));
-    const float2 s1 = make_float2(__uint2float_rn(S10), __uint2float_rn(S11));
-    const float2 s2 = make_float2(__uint2float_rn(S20), __uint2float_rn(S21));
-    const float2 nn2 = make_float2(nnf, nnf);
-    const float2 p = __fmul2_rn(make_float2(csum, csum), s1);
-    const float2 nx = __ffma2_rn(nn2, d, neg2(p));
-    const float2 tn = __ffma2_rn(nn2, d, p);
-    float2 vx, tv;
-    if (measure == AR_NCC) {
-        vx = s2;
-        tv = s2;
-    } else {
-        const float2 q = __fmul2_rn(s1, s1);
-        vx = __ffma2_rn(nn2, s2, neg2(q));
-        tv = __ffma2_rn(nn2, s2, q);
-    }
-    const float2 ev = __fmul2_rn(make_float2(3.5762786865234375e-07f, 3.5762786865234375e-07f), tv);
-    const float2 ev64 = __fmul2_rn(make_float2(64.0f, 64.0f), ev);
-    const bool ok0 = vx.x > ev64.x, ok1 = vx.y > ev64.y;
-    const float2 r = make_float2(rsqrtf(ok0 ? vx.x : 1.0f), rsqrtf(ok1 ? vx.y : 1.0f));
-    const float2 est = __fmul2_rn(__fmul2_rn(nx, r), make_float2(k, k));
-    const float2 rel = __ffma2_rn(ev, __fmul2_rn(r, r),
-                                  make_float2(9.5367431640625e-07f, 9.5367431640625e-07f));
-    const float2 b = __fadd2_rn(
-        __ffma2_rn(make_float2(fabsf(est.x), fabsf(est.y)), __fmul2_rn(make_float2(2.0f, 2.0f), rel),
-                   __fmul2_rn(__fmul2_rn(tn, r), make_float2(k7, k7))),
-        make_float2(1e-30f, 1e-30f));
-    const float qn = __int_as_float(0x7fc00000);
-    *bound = make_float2(ok0 ? b.x : 0.0f, ok1 ? b.y : 0.0f);
-    return make_float2(ok0 ? est.x : qn, ok1 ? est.y : qn);
-}
 
 // Rows of the chip operand that block q's product needs: operand row e holds offset
 // u = e - NB + 16 (surface row i = 16 q + u), and only surface rows 0 <= i < nr are read, so
@@ -1630,10 +1600,7 @@ __device__ __forceinline__ void staged_chip_stats(const uint8_t* s_P, int PC, in
 
 // REG: every surface of the pass has at most 64 rows and 64 columns (M = 64), so one 16x256b
 // read per warp covers it and each thread keeps its 16 numerators and upper bounds in
-// registers through both passes. Otherwise the numerators go to shared memory and both passes
-// run over the surface in flattened order, four values per thread and step, so that every warp
-// has work even when the surface's columns fill only two or three of the M = 128 accumulator's
-// lane quarters.
+// registers through both passes. Otherwise each pass reads the numerators from Tensor Memory.
 template <bool REG>
 __global__ void __launch_bounds__(kTcThreads, 2) k_corr_tc(const TcArgs A) {
     extern __shared__ __align__(1024) unsigned char smem_tc[];
@@ -1642,23 +1609,23 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_corr_tc(const TcArgs A) {
     __shared__ int s_slot;
     __shared__ int s_ncand;
     __shared__ uint32_t s_pd[25];
-    __shared__ float s_fmax[kTcThreads / 32];
+    __shared__ float s_fmax[kTcThreads / 32], s_sec[kTcThreads / 32];
+    __shared__ int s_at[kTcThreads / 32];
     __shared__ unsigned long long s_isum[2][2];
     uint8_t* s_E = smem_tc + A.off_E;
     uint8_t* s_W = smem_tc + A.off_W;
-    uint8_t* s_T = smem_tc + A.off_T;
     uint8_t* s_P = smem_tc + A.off_P;
     uint32_t* s_V1 = reinterpret_cast<uint32_t*>(smem_tc + A.off_V);
-    uint32_t* s_S1 = reinterpret_cast<uint32_t*>(smem_tc + A.off_S1);
-    uint32_t* s_S2 = reinterpret_cast<uint32_t*>(smem_tc + A.off_S2);
+    uint2* s_S = reinterpret_cast<uint2*>(smem_tc + A.off_S1);  // box sums of W, of W^2
+    float* s_R = reinterpret_cast<float*>(smem_tc + A.off_R);
     uint32_t* s_num = reinterpret_cast<uint32_t*>(smem_tc + A.off_num);
     float* s_est = reinterpret_cast<float*>(smem_tc + A.off_est);
     double* s_red = reinterpret_cast<double*>(smem_tc + A.off_red);
 
     const int tid = threadIdx.x, bd = blockDim.x;
     const int lane = tid & 31, warp = tid >> 5, nwarps = bd >> 5;
-    // Threads issuing the products (only plans of the register epilogue take four).
-    const int NI = REG ? A.issuers : 2;
+    // Threads issuing the products (four where REG has the SM to itself).
+    const int NI = A.issuers;
     const int64_t NR = A.nrows + 2 * A.pady, NC = A.ncols + 2 * A.padx;
     const double shx = static_cast<double>(A.padx) + 0.5;
     const double shy = static_cast<double>(A.pady) + 0.5;
@@ -1688,13 +1655,13 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_corr_tc(const TcArgs A) {
     TC_PHASE_INIT
 
     // Each CTA takes a contiguous run of points: consecutive points of a grid column have the
-    // same window columns one grid step lower, so most of their box sums carry over. s_S1 / s_S2
-    // are rings of NRS rows per column: surface row i of the held point is stored at row
+    // same window columns one grid step lower, so most of their box sums carry over. s_S
+    // is a ring of NRS rows per column: surface row i of the held point is stored at row
     // (i + rbase) mod NRS, and carrying the sums down by `sh` rows advances rbase.
     const int64_t per = (A.pts.n + gridDim.x - 1) / gridDim.x;
     const int64_t kbeg = static_cast<int64_t>(blockIdx.x) * per;
     const int64_t kend = min(A.pts.n, kbeg + per);
-    bool held = false;  // s_S1 / s_S2 hold the sums of the geometry h_*
+    bool held = false;  // s_S holds the sums of the geometry h_*
     int64_t h_wr = 0, h_wc = 0;
     int h_ch = 0, h_cw = 0, h_nr = 0, h_nc = 0;
     int rbase = 0;
@@ -1849,14 +1816,11 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_corr_tc(const TcArgs A) {
         if (tid == 0 && carry) atomicAdd(&g_tc_phase[14], 1ull);
 #endif
 
-        // Window blocks W'[16 q + r][x] (x < XS) from 16 image rows at base_r + 16 q, and the
-        // same window transposed, s_T[row][x], for the box sums (the blocks from the one that
-        // holds window row iA: the rows the box sums read).
+        // Window blocks W'[16 q + r][x] (x < XS) from 16 image rows at base_r + 16 q.
         const int64_t delta = ((win_r % 16) + 16) % 16;
         const int64_t base_r = win_r - delta;
         const int Q = static_cast<int>((delta + ch + nr - 1 + 15) / 16);
         const int XW = cw + nc - 1;
-        const int qT = static_cast<int>((delta + iA) >> 4);
         // A block is one aligned 16-byte load when the image's columns are 16-byte aligned (row
         // counts divisible by 16), otherwise two aligned loads and a byte shift.
         // A task is block q of column x (consecutive threads on consecutive columns); each thread
@@ -1880,111 +1844,44 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_corr_tc(const TcArgs A) {
                     const int q = tq[u], x = tx[u];
                     const uint4 v = col16_finish(L[u]);
                     *reinterpret_cast<uint4*>(s_W + q * A.QS + x * 16) = v;
-                    if (A.big != 2 && x < XW && q >= qT) {
-                        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                        for (int t = 0; t < 16; ++t)
-                            s_T[(16 * q + t) * A.XT + x] = static_cast<uint8_t>(w[t >> 2] >> (8 * (t & 3)));
-                    }
                 }
             }
         }
-        __syncthreads();  // s_P, s_W, s_T complete
+        __syncthreads();  // s_P, s_W complete
         TC_PHASE(4)
 
-        // Box sums of W and W^2 (integral_both!, boxsum, src/integral.jl:141-170, 244-247) as
-        // exact integers: V[i][x] sums ch rows down column x, S[j][i] sums cw columns of V.
-        // They run while the tensor core works on the first chunk, or, when the chip operand
-        // comes in several chunks that reuse their space, before it. Only surface rows
-        // iA .. nr - 1 are computed (the others carried over), into ring rows.
-        // Threads 0 .. kBT - 1 (named barrier 1): the warps below the issuing ones.
-        auto box_sums = [&](const int kBT) {
-            uint32_t* s_V2 = s_V1 + A.NRM * XW;
-            const int nrw = nr - iA;
-            // V: one round of tasks (column x, a run of rows), each an unrolled first sum with
-            // independent partials and a sliding update with the next values loaded ahead.
-            const int nseg = max(1, min((nrw + 7) / 8, kBT / XW));
-            const int seglen = (nrw + nseg - 1) / nseg;
-            for (int task = tid; task < XW * nseg; task += kBT) {
-                const int x = task % XW, seg = task / XW;
-                const int i0 = iA + seg * seglen, i1 = min(i0 + seglen, nr);
-                if (i0 >= i1) continue;
-                const uint8_t* col = s_T + static_cast<int>(delta) * A.XT + x;
-                uint32_t p1[4] = {0, 0, 0, 0}, p2[4] = {0, 0, 0, 0};
-                int a = 0;
-                for (; a + 4 <= ch; a += 4) {
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const uint32_t w = col[(i0 + a + u) * A.XT];
-                        p1[u] += w;
-                        p2[u] += w * w;
-                    }
-                }
-                for (; a < ch; ++a) {
-                    const uint32_t w = col[(i0 + a) * A.XT];
-                    p1[0] += w;
-                    p2[0] += w * w;
-                }
-                uint32_t h1 = (p1[0] + p1[1]) + (p1[2] + p1[3]);
-                uint32_t h2 = (p2[0] + p2[1]) + (p2[2] + p2[3]);
-                uint32_t wo = col[i0 * A.XT], wn = col[(i0 + ch) * A.XT];
-                for (int i = i0; i < i1; ++i) {
-                    s_V1[i * XW + x] = h1;
-                    s_V2[i * XW + x] = h2;
-                    if (i + 1 < i1) {
-                        const uint32_t wo2 = col[(i + 1) * A.XT], wn2 = col[(i + 1 + ch) * A.XT];
-                        h1 = h1 + wn - wo;
-                        h2 = h2 + wn * wn - wo * wo;
-                        wo = wo2;
-                        wn = wn2;
-                    }
-                }
+        // The reciprocal roots of two values' variance terms (pass 1).
+        const float nnf = static_cast<float>(nnl);
+        auto recip2 = [&](uint2 a, uint2 b) {
+            const float2 s1 = make_float2(__uint2float_rn(a.x), __uint2float_rn(b.x));
+            const float2 s2 = make_float2(__uint2float_rn(a.y), __uint2float_rn(b.y));
+            float2 vx = s2;
+            if (A.measure != AR_NCC) {
+                const float2 q = __fmul2_rn(s1, s1), n2 = make_float2(nnf, nnf);
+                vx = __ffma2_rn(n2, s2, neg2(q));
+                const float2 tv = __ffma2_rn(n2, s2, q);
+                vx.x = tv.x > 2048.0f * vx.x ? -1.0f : vx.x;  // its root is NaN
+                vx.y = tv.y > 2048.0f * vx.y ? -1.0f : vx.y;
             }
-            asm volatile("bar.sync 1, %0;" ::"r"(kBT) : "memory");
-            // S: tasks (surface row i, a run of 16 columns), the same pattern along V's rows.
-            const int jseg = (nc + 15) >> 4;
-            for (int task = tid; task < nrw * jseg; task += kBT) {
-                const int i = iA + task % nrw, seg = task / nrw;
-                const int ri = ring(i);
-                const int j0 = seg << 4, j1 = min(j0 + 16, nc);
-                const uint32_t* v1 = s_V1 + i * XW;
-                const uint32_t* v2 = s_V2 + i * XW;
-                uint32_t q1[4] = {0, 0, 0, 0}, q2[4] = {0, 0, 0, 0};
-                int b = 0;
-                for (; b + 4 <= cw; b += 4) {
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        q1[u] += v1[j0 + b + u];
-                        q2[u] += v2[j0 + b + u];
-                    }
-                }
-                for (; b < cw; ++b) {
-                    q1[0] += v1[j0 + b];
-                    q2[0] += v2[j0 + b];
-                }
-                uint32_t g1 = (q1[0] + q1[1]) + (q1[2] + q1[3]);
-                uint32_t g2 = (q2[0] + q2[1]) + (q2[2] + q2[3]);
-                for (int j = j0; j < j1; ++j) {
-                    s_S1[j * A.NRS + ri] = g1;
-                    s_S2[j * A.NRS + ri] = g2;
-                    if (j + 1 < j1) {
-                        g1 = g1 + v1[j + cw] - v1[j];
-                        g2 = g2 + v2[j + cw] - v2[j];
-                    }
-                }
-            }
+            return make_float2(a.y == 0u ? 0.0f : rsqrtf(vx.x), b.y == 0u ? 0.0f : rsqrtf(vx.y));
         };
-        // The same sums in stripes of A.VR surface rows, for geometries whose column sums of every
-        // surface row do not fit beside the window (chips of 64 px and up with surfaces beyond
-        // 64 x 64). Column sums of a stripe straight from the 16-byte window blocks (no transposed
+        const bool roots = !REG && A.roots;  // s_R holds them, carried like the box sums
+
+        // Box sums of W and W^2 (integral_both!, boxsum, src/integral.jl:141-170, 244-247) as
+        // exact integers, in stripes of A.VR surface rows, by the threads below kBT (named barrier
+        // 1). They run while the tensor core works on the chip operand, or, when that comes in
+        // chunks that share the stripe's space, before it. Only surface rows iA .. nr - 1 are
+        // computed (the others carried over), into ring rows. Column sums of a stripe straight
+        // from the 16-byte window blocks (no transposed
         // copy): a thread per column, dp4a over the chip's rows for the stripe's first row, then a
         // slide of four rows at a time. Row sums of a stripe as prefix sums, a warp per row: a
         // difference of two prefixes is exact modulo 2^32 and the sums are below 2^32.
-        auto box_sums_striped = [&]() {
+        auto box_sums = [&](const int kBT) {
+            auto bar_box = [&]() { asm volatile("bar.sync 1, %0;" ::"r"(kBT) : "memory"); };
             uint32_t* s_V2 = s_V1 + A.VR * A.XV;
             for (int is = iA; is < nr; is += A.VR) {
                 const int ie = min(is + A.VR, nr);
-                for (int x = tid; x < XW; x += kTcThreads) {
+                for (int x = tid; x < XW; x += kBT) {
                     const uint8_t* col = s_W + x * 16;
                     const int R0 = static_cast<int>(delta) + is, R1 = R0 + ch;
                     uint32_t h1 = 0u, h2 = 0u;
@@ -2035,8 +1932,8 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_corr_tc(const TcArgs A) {
                         }
                     }
                 }
-                __syncthreads();
-                for (int i = is + warp; i < ie; i += nwarps) {
+                bar_box();
+                for (int i = is + warp; i < ie; i += kBT >> 5) {
                     uint32_t* v1 = s_V1 + (i - is) * A.XV;
                     uint32_t* v2 = s_V2 + (i - is) * A.XV;
                     uint32_t c1 = 0u, c2 = 0u;
@@ -2067,18 +1964,18 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_corr_tc(const TcArgs A) {
                     __syncwarp();
                     const int ri = ring(i);
                     for (int j = lane; j < nc; j += 32) {
-                        s_S1[j * A.NRS + ri] = v1[j + cw - 1] - (j > 0 ? v1[j - 1] : 0u);
-                        s_S2[j * A.NRS + ri] = v2[j + cw - 1] - (j > 0 ? v2[j - 1] : 0u);
+                        const uint32_t s1 = v1[j + cw - 1] - (j > 0 ? v1[j - 1] : 0u);
+                        const uint32_t s2 = v2[j + cw - 1] - (j > 0 ? v2[j - 1] : 0u);
+                        s_S[j * A.NRS + ri] = make_uint2(s1, s2);
+                        if (roots) s_R[j * A.NRS + ri] = recip2(make_uint2(s1, s2), make_uint2(s1, s2)).x;
                     }
                 }
-                __syncthreads();  // the next stripe, or the chip chunks, overwrite the sums
+                if (ie < nr) bar_box();  // the next stripe overwrites the sums
             }
         };
-        if (A.big == 2) {
-            box_sums_striped();
-        } else if (A.big) {
-            if (warp < nwarps - NI) box_sums(kTcThreads - 32 * NI);
-            __syncthreads();  // the chip chunks overwrite s_T and s_V
+        if (A.big) {
+            box_sums(kTcThreads);
+            __syncthreads();  // the chip chunks overwrite the stripe
         }
 
         const int nchunk = (cw + A.BC - 1) / A.BC;
@@ -2137,9 +2034,8 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_corr_tc(const TcArgs A) {
             // Lane 0 of each of the last NI warps issues the products of a share of the
             // chunk's chip column pairs into its own accumulator (one thread's MMAs run one after
             // another, so the products of one point are spread over two or four threads).
-            if (REG ? (lane == 0 && warp >= nwarps - NI)
-                    : (tid == kTcThreads - 32 || tid == kTcThreads - 64)) {
-                const int stream = REG ? nwarps - 1 - warp : (tid == kTcThreads - 32 ? 0 : 1);
+            if (lane == 0 && warp >= nwarps - NI) {
+                const int stream = nwarps - 1 - warp;
                 tc::fence_after_sync();
                 const uint32_t sW = tc::smem_u32(s_W), sE = tc::smem_u32(s_E);
                 const int p0 = b0 / 2, p1 = b1 / 2;
@@ -2187,12 +2083,28 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_corr_tc(const TcArgs A) {
             A.measure == AR_NCC ? __drcp_rn(__dmul_rn(cnorm, nn))
                                 : __drcp_rn(__dmul_rn(cnorm, __dsqrt_rn(nn))));
         const float kk7 = 4.172325134277344e-07f * kk;  // 7u k
-        const float nnf = static_cast<float>(nnl);
         const float csf = static_cast<float>(csum_d);
         const int quarter = warp & 3, half = warp >> 2;
-        const uint32_t col0 = 0u;
-        float lmax = -INFINITY;
+        unsigned long long best = 0ull;
+        int pi = 0, pj = 0;  // the peak
+        // The peak or its 5 x 5 patch (all inside the surface): the numerators of the output.
+        const bool single = A.up == 1 || nr < 5 || nc < 5;
+        const int span = single ? 1 : 5;
+        int pi0 = 0, pj0 = 0;
+        auto patch_at = [&](int i, int j) {
+            pi = i;
+            pj = j;
+            pi0 = single ? pi : min(max(pi - 2, 0), max(nr - 5, 0));
+            pj0 = single ? pj : min(max(pj - 2, 0), max(nc - 5, 0));
+        };
+        auto patch_of = [&](unsigned long long key) {
+            unsigned rm = 0;
+            float pv = 0.0f;
+            if (key_decode(key, &rm, &pv)) patch_at(static_cast<int>(rm / nc), static_cast<int>(rm % nc));
+            else patch_at(0, 0);
+        };
         if constexpr (REG) {
+            float lmax = -INFINITY;
             // One read per warp: value v of this thread is surface row
             // i = 32 half + 8 (v / 4) + 2 (lane % 4) + v % 2, column j = 16 quarter + lane / 4
             // (+ 8 when v % 4 >= 2). Registers keep its numerator and its upper bound.
@@ -2202,7 +2114,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_corr_tc(const TcArgs A) {
             float upb[16];
             uint32_t vm = 0u;  // values of this thread inside the surface
             if (32 * half < nr) {
-                const uint32_t base = taddr + (static_cast<uint32_t>(32 * quarter) << 16) + col0 +
+                const uint32_t base = taddr + (static_cast<uint32_t>(32 * quarter) << 16) +
                                       static_cast<uint32_t>(32 * half);
                 uint32_t dv1[16];
                 tc::tmem_ld16dp(base, dv);
@@ -2224,7 +2136,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_corr_tc(const TcArgs A) {
                         vm |= 1u << v;
                         const int o = j * A.NRS + ring(i);
                         float bnd;
-                        const float est = tc_estimate(dv[v], s_S1[o], s_S2[o], nnf, csf, kk, kk7,
+                        const float est = tc_estimate(dv[v], s_S[o].x, s_S[o].y, nnf, csf, kk, kk7,
                                                       A.measure, &bnd);
                         upb[v] = est + bnd;
                         lmax = fmaxf(lmax, est - bnd);
@@ -2254,11 +2166,10 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_corr_tc(const TcArgs A) {
             }
             __syncthreads();
             const int ncand = s_ncand;
-            unsigned long long best = 0ull;
             for (int c = tid; c < ncand; c += bd) {
                 const int i = static_cast<int>(s_cI[c] >> 16), j = static_cast<int>(s_cI[c] & 0xFFFFu);
                 const int o = j * A.NRS + ring(i);
-                const float x = tc_exact(s_cD[c], s_S1[o], s_S2[o], mean, nn, cnorm, A.measure);
+                const float x = tc_exact(s_cD[c], s_S[o].x, s_S[o].y, mean, nn, cnorm, A.measure);
                 const unsigned long long key = argmax_key(x, static_cast<unsigned>(i * nc + j));
                 best = key > best ? key : best;
             }
@@ -2277,245 +2188,179 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_corr_tc(const TcArgs A) {
                 for (int e = tid; e < nr * nc; e += bd) {
                     const int o = (e / nr) * A.NRS + (e % nr);
                     const int os = (e / nr) * A.NRS + ring(e % nr);
-                    so[e] = tc_exact(s_num[o], s_S1[os], s_S2[os], mean, nn, cnorm, A.measure);
+                    so[e] = tc_exact(s_num[o], s_S[os].x, s_S[os].y, mean, nn, cnorm, A.measure);
                 }
             }
-            unsigned rm = 0;
-            float pv = 0.0f;
-            int pi = 0, pj = 0;
-            if (key_decode(best, &rm, &pv)) {
-                pi = static_cast<int>(rm / nc);
-                pj = static_cast<int>(rm % nc);
-            }
-            const bool single = A.up == 1 || nr < 5 || nc < 5;
-            // The numerators of the output: the peak, or the 5 x 5 patch (all inside the surface).
-            const int pi0 = single ? pi : min(max(pi - 2, 0), max(nr - 5, 0));
-            const int pj0 = single ? pj : min(max(pj - 2, 0), max(nc - 5, 0));
-            const int span = single ? 1 : 5;
+            patch_of(best);
 #pragma unroll
             for (int v = 0; v < 16; ++v) {
                 const int a = ib0 + 8 * (v >> 2) + (v & 1) - pi0, b = jb0 + ((v & 2) ? 8 : 0) - pj0;
                 if (a >= 0 && a < span && b >= 0 && b < span && ((vm >> v) & 1u)) s_pd[b * 5 + a] = dv[v];
             }
-            __syncthreads();
-            if (single) {
-                if (tid == 0) {
-                    const int o = pj * A.NRS + ring(pi);
-                    A.out.dx[k] = __double2float_rn(
-                        __dadd_rn(static_cast<double>(pj - static_cast<int>(prx)), A.pts.dx0[k]));
-                    A.out.dy[k] = __double2float_rn(
-                        __dadd_rn(static_cast<double>(pi - static_cast<int>(pry)), A.pts.dy0[k]));
-                    A.out.corr[k] = tc_exact(s_pd[0], s_S1[o], s_S2[o], mean, nn, cnorm, A.measure);
-                }
-            } else {
-                const int slot = s_slot;
-                if (tid < 25) {
-                    const int a = tid % 5, b = tid / 5;
-                    const int o = (pj0 + b) * A.NRS + ring(pi0 + a);
-                    A.sub_patch[static_cast<int64_t>(slot) * 25 + tid] =
-                        tc_exact(s_pd[tid], s_S1[o], s_S2[o], mean, nn, cnorm, A.measure);
-                }
-                if (tid == 0) {
-                    A.sub_point[slot] = k;
-                    A.sub_origin[2 * slot] = pi0;
-                    A.sub_origin[2 * slot + 1] = pj0;
-                }
-            }
-            TC_PHASE(10)
-            TC_PHASE_POINT
-            continue;
-        }
-        // The surface's values in flattened order e = i + nr j: thread t starts at e = t and
-        // steps by kTcThreads (row and column advanced without a division).
-        const int ne = nr * nc;
-        const int fj0 = tid / nr, fi0 = tid - fj0 * nr;
-        const int fdj = kTcThreads / nr, fdi = kTcThreads - fdj * nr;
-        auto fstep = [&](int& i, int& j) {
-            i += fdi;
-            j += fdj;
-            if (i >= nr) {
-                i -= nr;
-                ++j;
-            }
-        };
-        auto take = [&](uint32_t d, int i, int j) {
-            if (j < nc && i < nr) {
-                const int o = j * A.NRS + i;
-                const int os = j * A.NRS + ring(i);
-                float bnd;
-                const float est = tc_estimate(d, s_S1[os], s_S2[os], nnf, csf, kk, kk7, A.measure, &bnd);
-                s_num[o] = d;
-                s_est[o] = est + bnd;
-                lmax = fmaxf(lmax, est - bnd);
-            }
-        };
-        if (A.MT == 64) {
-            for (int i0 = 32 * half; i0 < nr; i0 += 64) {
-                uint32_t r[16], r1[16];
-                const uint32_t base = taddr + (static_cast<uint32_t>(32 * quarter) << 16) + col0 +
-                                      static_cast<uint32_t>(i0);
-                tc::tmem_ld16dp(base, r);
-                tc::tmem_ld16dp(base + acc1, r1);
-                tc::tmem_wait_ld();
-#pragma unroll
-                for (int v = 0; v < 16; ++v) r[v] += r1[v];
-                for (int s = 2; s < NI; ++s) {
-                    tc::tmem_ld16dp(base + static_cast<uint32_t>(s) * acc1, r1);
-                    tc::tmem_wait_ld();
-#pragma unroll
-                    for (int v = 0; v < 16; ++v) r[v] += r1[v];
-                }
-#pragma unroll
-                for (int v = 0; v < 16; ++v)
-                    take(r[v], i0 + 8 * (v >> 2) + 2 * (lane & 3) + (v & 1),
-                         16 * quarter + (lane >> 2) + ((v & 2) ? 8 : 0));
-            }
         } else {
-            // M = 128: accumulator row j is lane j; thread = row 32 q + lane, 16 columns. Only
-            // the lane quarters below nc hold surface columns (for nc <= 96, two or three of
-            // the four), so their warps move the numerators to shared memory and the estimates
-            // are spread over all warps: warp w takes columns w, w + 8, ..., lanes the rows.
-            if (32 * quarter < nc) {
-                const int j = 32 * quarter + lane;
-                for (int i0 = 16 * half; i0 < nr; i0 += 32) {
-                    uint32_t r[16], r1[16];
-                    const uint32_t base = taddr + (static_cast<uint32_t>(32 * quarter) << 16) +
-                                          col0 + static_cast<uint32_t>(i0);
-                    tc::tmem_ld16(base, r);
-                    tc::tmem_ld16(base + acc1, r1);
-                    tc::tmem_wait_ld();
+            // Numerators out of Tensor Memory, of surface rows ilo .. ihi - 1 and columns
+            // jlo .. jhi - 1 and more beside them: fn(two numerators, the even row of the first, column),
+            // rows (an even number) and columns beyond the surface included. M = 128: accumulator row j is lane j, a thread reads 16
+            // columns; M = 64 as above.
+            auto visit = [&](int ilo, int ihi, int jlo, int jhi, auto&& fn) {
+                uint32_t r[16], r1[16];
+                if (A.MT == 64) {
+                    if (16 * quarter >= jhi || 16 * quarter + 16 <= jlo) return;
+                    for (int i0 = 32 * half; i0 < nr; i0 += 64) {
+                        if (i0 >= ihi || i0 + 32 <= ilo) continue;
+                        const uint32_t base = taddr + (static_cast<uint32_t>(32 * quarter) << 16) +
+                                              static_cast<uint32_t>(i0);
+                        tc::tmem_ld16dp(base, r);
+                        for (int s = 1; s < NI; ++s) {
+                            tc::tmem_ld16dp(base + static_cast<uint32_t>(s) * acc1, r1);
+                            tc::tmem_wait_ld();
 #pragma unroll
-                    for (int m = 0; m < 16; ++m) r[m] += r1[m];
-                    for (int s = 2; s < NI; ++s) {
-                        tc::tmem_ld16(base + static_cast<uint32_t>(s) * acc1, r1);
-                        tc::tmem_wait_ld();
+                            for (int v = 0; v < 16; ++v) r[v] += r1[v];
+                        }
 #pragma unroll
-                        for (int m = 0; m < 16; ++m) r[m] += r1[m];
+                        for (int v = 0; v < 16; v += 2)
+                            fn(r[v], r[v + 1], i0 + 8 * (v >> 2) + 2 * (lane & 3),
+                               16 * quarter + (lane >> 2) + ((v & 2) ? 8 : 0));
                     }
-                    if (j < nc) {
+                } else {
+                    if (32 * quarter >= jhi || 32 * quarter + 32 <= jlo) return;
+                    for (int i0 = 16 * half; i0 < nr; i0 += 32) {
+                        if (i0 >= ihi || i0 + 16 <= ilo) continue;
+                        const uint32_t base = taddr + (static_cast<uint32_t>(32 * quarter) << 16) +
+                                              static_cast<uint32_t>(i0);
+                        tc::tmem_ld16(base, r);
+                        for (int s = 1; s < NI; ++s) {
+                            tc::tmem_ld16(base + static_cast<uint32_t>(s) * acc1, r1);
+                            tc::tmem_wait_ld();
 #pragma unroll
-                        for (int m = 0; m < 16; ++m)
-                            if (i0 + m < nr) s_num[j * A.NRS + i0 + m] = r[m];
+                            for (int v = 0; v < 16; ++v) r[v] += r1[v];
+                        }
+#pragma unroll
+                        for (int v = 0; v < 16; v += 2) fn(r[v], r[v + 1], i0 + v, 32 * quarter + lane);
                     }
+                }
+            };
+            // The estimate of a value, times kz, and the error bound `bu` of all of them as in
+            // k_corr_tc2 (its pass 1): reciprocal roots carried with the box sums, no bound a value,
+            // no surface in shared memory. With a bound for each value, numerators and upper bounds
+            // staged for a second pass over all of them, these two passes took 11 k of a point's
+            // 31.7 k cycles at chip 32, surface 88 x 88.
+            auto estimate = [&](uint32_t d0, uint32_t d1, int o0, int o1) {
+                const uint2 a = s_S[o0], b = s_S[o1];
+                const float2 s1 = make_float2(__uint2float_rn(a.x), __uint2float_rn(b.x));
+                const float2 nx = __ffma2_rn(make_float2(nnf, nnf),
+                                             make_float2(__uint2float_rn(d0), __uint2float_rn(d1)),
+                                             neg2(__fmul2_rn(make_float2(csf, csf), s1)));
+                return __fmul2_rn(nx, roots ? make_float2(s_R[o0], s_R[o1]) : recip2(a, b));
+            };
+            const float u24 = 6.0200e-08f;  // 1.01 x 2^-24
+            const float kz = sqrtf(static_cast<float>(sq) * nnf);
+            const float kc = sqrtf(nnf * static_cast<float>(sq + csum_d * mean));
+            const float bu = A.measure == AR_NCC ? u24 * sqrtf(nnf) * (20.0f * kz + 5.0f * kc)
+                                                 : u24 * (3400.0f * kz + 160.0f * kc);
+            float sum = 0.0f;                          // NaN when an estimate was not made
+            float own = -INFINITY, own2 = -INFINITY;  // this thread's two largest estimates
+            int at = 0;                               // where the largest is
+            // The ring places of rows i and i + 1 (of the last two for rows beyond the surface).
+            auto places = [&](int i, int j, int* o0, int* o1) {
+                const unsigned r = static_cast<unsigned>(min(i, nr - 2) + rbase);
+                const unsigned n = static_cast<unsigned>(A.NRS), base = min(j, nc - 1) * n;
+                *o0 = static_cast<int>(base + min(r, r - n));
+                *o1 = static_cast<int>(base + min(r + 1u, r + 1u - n));
+            };
+            visit(0, nr, 0, nc, [&](uint32_t d0, uint32_t d1, int i, int j) {
+                const bool in = i < nr && j < nc;
+                int o0, o1;
+                places(i, j, &o0, &o1);
+                const float2 e = estimate(d0, d1, o0, o1);
+                sum += in ? e.x + e.y : 0.0f;
+                const float hi = in ? fmaxf(e.x, e.y) : -INFINITY, lo = in ? fminf(e.x, e.y) : -INFINITY;
+                own2 = fmaxf(own2, fmaxf(lo, fminf(own, hi)));
+                at = hi > own ? ((e.y > e.x ? i + 1 : i) << 16) | j : at;
+                own = fmaxf(own, hi);
+            });
+            {
+                const float top = warp_max(own);
+                const unsigned who = __ballot_sync(kFull, own == top && own > -INFINITY);
+                const int first = who ? __ffs(who) - 1 : 0;
+                const float sec = warp_max(isnan(sum) ? INFINITY : lane == first ? own2 : own);
+                if (lane == first) {
+                    s_fmax[warp] = top;
+                    s_sec[warp] = sec;
+                    s_at[warp] = at;
                 }
             }
             __syncthreads();
-            // Four values per thread and step, their loads issued before the (paired) arithmetic.
-            int fi = fi0, fj = fj0;
-            for (int e = tid; e < ne; e += 4 * kTcThreads) {
-                int o[4], os[4];
-                bool in[4];
-                uint32_t d[4], s1[4], s2[4];
+            TC_PHASE(8)
+            // Is the largest estimate more than the bound above every other?
+            constexpr int kW = kTcThreads / 32;
+            const float wt = lane < kW ? s_fmax[lane] : -INFINITY;
+            const float M = warp_max(wt);
+            const float cut = M - 2.0f * bu;
+            const int mw = __ffs(__ballot_sync(kFull, wt == M)) - 1;
+            const bool unique =
+                M > -INFINITY && !__any_sync(kFull, lane < kW && (!(s_sec[lane & (kW - 1)] < cut) ||
+                                                                  (lane != mw && !(wt < cut))));
+            if (unique) {
+                // Every other value is below this one: it is the strict (so the first) maximum.
+                patch_at(s_at[mw] >> 16, s_at[mw] & 0xFFFF);
+            } else {
+                // The values whose estimate is within the bounds of the largest (or was not made),
+                // exactly.
+                visit(0, nr, 0, nc, [&](uint32_t d0, uint32_t d1, int i, int j) {
+                    if (i >= nr || j >= nc) return;
+                    int o[2];
+                    places(i, j, &o[0], &o[1]);
+                    const float2 e = estimate(d0, d1, o[0], o[1]);
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    in[u] = e + u * kTcThreads < ne;
-                    o[u] = fj * A.NRS + fi;
-                    os[u] = fj * A.NRS + ring(fi);
-                    fstep(fi, fj);
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    d[u] = in[u] ? s_num[o[u]] : 0u;
-                    s1[u] = in[u] ? s_S1[os[u]] : 0u;
-                    s2[u] = in[u] ? s_S2[os[u]] : 0u;
-                }
-                float2 b01, b23;
-                const float2 e01 = tc_estimate2(d[0], d[1], s1[0], s1[1], s2[0], s2[1], nnf, csf,
-                                                kk, kk7, A.measure, &b01);
-                const float2 e23 = tc_estimate2(d[2], d[3], s1[2], s1[3], s2[2], s2[3], nnf, csf,
-                                                kk, kk7, A.measure, &b23);
-                const float ev[4] = {e01.x, e01.y, e23.x, e23.y};
-                const float bv[4] = {b01.x, b01.y, b23.x, b23.y};
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    if (in[u]) {
-                        s_est[o[u]] = ev[u] + bv[u];
-                        lmax = fmaxf(lmax, ev[u] - bv[u]);
+                    for (int u = 0; u < 2; ++u) {
+                        if ((u ? e.y : e.x) < cut) continue;
+                        const float x = tc_exact(u ? d1 : d0, s_S[o[u]].x, s_S[o[u]].y, mean, nn, cnorm, A.measure);
+                        const unsigned long long key = argmax_key(x, static_cast<unsigned>((i + u) * nc + j));
+                        best = key > best ? key : best;
                     }
-                }
+                });
+                best = block_max_u64(best, reinterpret_cast<unsigned long long*>(s_red));
+                patch_of(best);
             }
+            TC_PHASE(9)
+            if (A.flops && tid == 0)
+                atomicAdd(A.flops, 2ull * static_cast<unsigned long long>(ch) * cw * nr * nc);
+            if (A.surf_out) {
+                float* so = A.surf_out + k * static_cast<int64_t>(A.NRM) * A.NCM;
+                visit(0, nr, 0, nc, [&](uint32_t d0, uint32_t d1, int i, int j) {
+                    if (i >= nr || j >= nc) return;
+                    int o0, o1;
+                    places(i, j, &o0, &o1);
+                    so[j * nr + i] = tc_exact(d0, s_S[o0].x, s_S[o0].y, mean, nn, cnorm, A.measure);
+                    so[j * nr + i + 1] = tc_exact(d1, s_S[o1].x, s_S[o1].y, mean, nn, cnorm, A.measure);
+                });
+            }
+            visit(pi0, pi0 + span, pj0, pj0 + span, [&](uint32_t d0, uint32_t d1, int i, int j) {
+                const int a = i - pi0, b = j - pj0;
+                if (i < nr && b >= 0 && b < span) {
+                    if (a >= 0 && a < span) s_pd[b * 5 + a] = d0;
+                    if (a + 1 >= 0 && a + 1 < span) s_pd[b * 5 + a + 1] = d1;
+                }
+            });
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) lmax = fmaxf(lmax, __shfl_xor_sync(kFull, lmax, o));
-        if (lane == 0) s_fmax[warp] = lmax;
         __syncthreads();
-        TC_PHASE(8)
-        float M = s_fmax[0];
-        for (int w = 1; w < kTcThreads / 32; ++w) M = fmaxf(M, s_fmax[w]);
-        // M: the largest lower bound of any value. A value whose upper bound is below it is
-        // strictly below some other value: it cannot be the (first) maximum.
-
-        // Pass 2: exact values where the upper bound reaches M; the peak key. The same flattened
-        // order, four values per thread and step.
-        unsigned long long best = 0ull;
-        {
-            int fi = fi0, fj = fj0;
-            for (int e = tid; e < ne; e += 4 * kTcThreads) {
-                int o[4], ii[4], jj[4];
-                bool in[4];
-                float upb[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    in[u] = e + u * kTcThreads < ne;
-                    ii[u] = fi;
-                    jj[u] = fj;
-                    o[u] = fj * A.NRS + fi;
-                    fstep(fi, fj);
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) upb[u] = in[u] ? s_est[o[u]] : 0.0f;
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    if (!in[u] || (!(upb[u] >= M) && !isnan(upb[u]))) continue;
-                    const int os = jj[u] * A.NRS + ring(ii[u]);
-                    const float v =
-                        tc_exact(s_num[o[u]], s_S1[os], s_S2[os], mean, nn, cnorm, A.measure);
-                    const unsigned long long key =
-                        argmax_key(v, static_cast<unsigned>(ii[u] * nc + jj[u]));
-                    best = key > best ? key : best;
-                }
-            }
-        }
-        best = block_max_u64(best, reinterpret_cast<unsigned long long*>(s_red));
-        TC_PHASE(9)
-        if (A.flops && tid == 0)
-            atomicAdd(A.flops, 2ull * static_cast<unsigned long long>(ch) * cw * nr * nc);
-        if (A.surf_out) {
-            float* so = A.surf_out + k * static_cast<int64_t>(A.NRM) * A.NCM;
-            for (int e = tid; e < nr * nc; e += bd) {
-                const int o = (e / nr) * A.NRS + (e % nr);
-                const int os = (e / nr) * A.NRS + ring(e % nr);
-                so[e] = tc_exact(s_num[o], s_S1[os], s_S2[os], mean, nn, cnorm, A.measure);
-            }
-        }
-        unsigned rm = 0;
-        float pv = 0.0f;
-        int pi = 0, pj = 0;
-        if (key_decode(best, &rm, &pv)) {
-            pi = static_cast<int>(rm / nc);
-            pj = static_cast<int>(rm % nc);
-        }
-        if (A.up == 1 || nr < 5 || nc < 5) {
+        if (single) {
             if (tid == 0) {
-                const int o = pj * A.NRS + pi;
-                const int os = pj * A.NRS + ring(pi);
-                const float v = tc_exact(s_num[o], s_S1[os], s_S2[os], mean, nn, cnorm, A.measure);
+                const int o = pj * A.NRS + ring(pi);
                 A.out.dx[k] = __double2float_rn(
                     __dadd_rn(static_cast<double>(pj - static_cast<int>(prx)), A.pts.dx0[k]));
                 A.out.dy[k] = __double2float_rn(
                     __dadd_rn(static_cast<double>(pi - static_cast<int>(pry)), A.pts.dy0[k]));
-                A.out.corr[k] = v;
+                A.out.corr[k] = tc_exact(s_pd[0], s_S[o].x, s_S[o].y, mean, nn, cnorm, A.measure);
             }
         } else {
-            const int pi0 = min(max(pi - 2, 0), max(nr - 5, 0));
-            const int pj0 = min(max(pj - 2, 0), max(nc - 5, 0));
             const int slot = s_slot;
             if (tid < 25) {
                 const int a = tid % 5, b = tid / 5;
-                const int o = (pj0 + b) * A.NRS + (pi0 + a);
-                const int os = (pj0 + b) * A.NRS + ring(pi0 + a);
+                const int o = (pj0 + b) * A.NRS + ring(pi0 + a);
                 A.sub_patch[static_cast<int64_t>(slot) * 25 + tid] =
-                    tc_exact(s_num[o], s_S1[os], s_S2[os], mean, nn, cnorm, A.measure);
+                    tc_exact(s_pd[tid], s_S[o].x, s_S[o].y, mean, nn, cnorm, A.measure);
             }
             if (tid == 0) {
                 A.sub_point[slot] = k;
@@ -2545,11 +2390,13 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_corr_tc(const TcArgs A) {
 // aligned global loads), so block q of 16 rows meets surface rows i in [16 q - ch + 1,
 // 16 q + 15]: NB = 16 * ceil((ch + 15) / 16) rows of the chip operand E_b[u][r] = C[r - u, b]
 // (u = 16 - NB ... 15). A block's product lands at accumulator column 16 q + e - (NB - 16) for
-// its operand row e, so surface row i is column i and the products of three issuing threads
-// write three accumulators of round16(nr) columns. The box sums come from the 16-byte window
-// blocks: column sums V down ch rows per 16-row block of surface rows (dp4a for the first, a
-// sliding update for the rest), then row sums of V with 16-byte loads. Estimates stay in
-// registers; candidates and the patch get the reference's FP64 normalisation.
+// its operand row e, so surface row i is column i and the products of four issuing threads
+// (lane 0 of the last four of eight main warps) write four accumulators. The box sums come from
+// the 16-byte window blocks: column sums V down ch rows (dp4a for the first row, a sliding update
+// for the rest), then row sums. A fetch warp stages the next point's window and chip and a patch
+// warp writes the last point's patch while the main warps work on this one. Estimates stay in
+// registers; the patch, and the values the bound does not separate from the largest, get the
+// reference's FP64 normalisation.
 
 // A point's chip and window placement (src/points.jl:358-395 with the pass's padding and the
 // +0.5 shift, src/track.jl:128-138, 207-220) and whether it is searched at all.
@@ -4815,10 +4662,10 @@ size_t tmem_smem_floor(uint32_t cols, size_t static_smem) {
 }
 
 struct TcPlan {
-    int NB, QM, QS, PS, PC, XS, XT, NRS, NRM, NCM, CHM, CWM, BC, big, MT;
-    unsigned off_E, off_W, off_T, off_P, off_V, off_S1, off_S2, off_num, off_est, off_red;
+    int NB, QM, QS, PS, PC, XS, NRS, NRM, NCM, CHM, CWM, BC, big, MT;
+    unsigned off_E, off_W, off_P, off_V, off_S1, off_S2, off_R = 0, off_num, off_est, off_red;
     unsigned off_L = 0, off_rawW = 0, off_rawC = 0;
-    int XV = 0, VR = 0, acc1_col = 0, issuers = 2;
+    int XV = 0, VR = 0, roots = 0, acc1_col = 0, issuers = 2;
     uint32_t tmem_cols;
     size_t smem;
 };
@@ -4844,7 +4691,6 @@ bool plan_corr_tc2(const PassGeometry& g, size_t smem_cap, TcPlan* P) {
     P->PS = P->NB * 16;
     P->XS = 64 + cw;
     P->QS = P->XS * 16;
-    P->XT = 0;
     P->PC = round_up(kPadL + P->NB + 20, 16);
     P->NRS = nr | 1;
     P->XV = round_up(cw + nc - 1, 32) + 4;
@@ -4897,7 +4743,6 @@ bool plan_corr_tc2(const PassGeometry& g, size_t smem_cap, TcPlan* P) {
         while (off > cap && vr > 16) off = layout(vr = std::max(16, (vr - 1) & ~15));
         if (off <= cap) break;
     }
-    P->off_T = 0;
     P->BC = cw;
     P->big = 0;
     P->smem = off;
@@ -4996,11 +4841,15 @@ void four_issuers(TcPlan* P) {
 }
 
 // Shared-memory plan of k_corr_tc for a pass's largest geometry; false when the pass does not
-// fit the kernel (surface wider than 64 columns, more than 256 rows, chips taller than 226).
-// The whole chip operand and separate box-sum buffers when they fit ("overlap": the box sums
-// run beside the products); otherwise the box sums first and the chip operand in chunks of BC
-// columns in the space they used; where even that space is too small for the column sums of every
-// surface row (chips of 64 px and up with surfaces beyond 64 x 64), the box sums in stripes.
+// fit the kernel (surface wider than 128 columns, more than 256 rows, chips taller than 226).
+// [box sums of W and W^2][reciprocal roots][red][P][W][V of a stripe of surface rows][E]: with the
+// whole chip operand E beside the stripe the box sums run beside the products. Otherwise the box sums
+// come first and the chip operand in chunks of BC columns in the stripe's place, without the
+// roots (they would cost a chip-64, radius-48 pass a chunk more). Either in half of an SM's
+// shared memory comes before either in all of it: 1.24 ms with two CTAs and chunks against 1.55
+// with one and the whole operand (14 400 points, chip 32, radius 44). The list of candidates of
+// surfaces up to 64 x 64 takes the place of W, V and E once the products are done (P keeps its
+// zero padding between points).
 bool plan_corr_tc(const PassGeometry& g, size_t smem_cap, TcPlan* P) {
     const int ch = static_cast<int>(g.max_ch), cw = static_cast<int>(g.max_cw);
     const int nr = static_cast<int>(g.max_nr), nc = static_cast<int>(g.max_nc);
@@ -5016,7 +4865,7 @@ bool plan_corr_tc(const PassGeometry& g, size_t smem_cap, TcPlan* P) {
     P->PS = P->NB * 16;
     P->XS = P->MT + cw;
     P->QS = P->XS * 16;
-    P->XT = round_up(cw + nc - 1, 4) + 4;
+    P->XV = round_up(cw + nc - 1, 4);
     P->PC = round_up(kPadL + P->NB + 20, 16);
     P->NRS = nr | 1;
     // Two accumulators, each holding the columns of surface rows 0 .. nr + 15 (the products'
@@ -5031,107 +4880,62 @@ bool plan_corr_tc(const PassGeometry& g, size_t smem_cap, TcPlan* P) {
     auto a16 = [](size_t v) { return (v + 15) & ~size_t(15); };
     const size_t Eb = static_cast<size_t>(cw) * P->PS;
     const size_t Wb = static_cast<size_t>(P->QM) * P->QS;
-    const size_t Tb = a16(static_cast<size_t>(16 * P->QM) * P->XT);
     const size_t Pb = a16(static_cast<size_t>(cw) * P->PC);
-    const size_t Vb = a16(2ull * nr * (cw + nc - 1) * 4);
     const size_t nbytes = a16(static_cast<size_t>(nc) * P->NRS * 4);
     const size_t red = 3 * 32 * 8;
-    // Overlap layout: [E][W][T][P][V | num, upper bounds][S1][S2][red].
-    {
+    const size_t row = 2 * static_cast<size_t>(P->XV) * 4;
+    const bool listed = P->MT == 64 && nr <= 64;
+    auto front = [&](int roots) {
+        P->roots = roots;
         size_t off = 0;
-        P->off_E = 0;
-        off += Eb;
-        P->off_W = static_cast<unsigned>(off);
-        off += Wb;
-        P->off_T = static_cast<unsigned>(off);
-        off += Tb;
-        P->off_P = static_cast<unsigned>(off);
-        off += Pb;
-        P->off_V = static_cast<unsigned>(off);
-        P->off_num = P->off_V;
-        P->off_est = static_cast<unsigned>(off + nbytes);
-        off += std::max(Vb, 2 * nbytes);
-        P->off_S1 = static_cast<unsigned>(off);
+        P->off_S1 = 0;
         off += nbytes;
         P->off_S2 = static_cast<unsigned>(off);
         off += nbytes;
+        P->off_R = static_cast<unsigned>(off);
+        off += roots ? nbytes : 0;
         P->off_red = static_cast<unsigned>(off);
-        off += red;
-        if (off <= smem_cap) {
-            P->smem = off;
+        off = a16(off + red);
+        P->off_P = static_cast<unsigned>(off);
+        off += Pb;
+        P->off_W = P->off_num = static_cast<unsigned>(off);
+        P->off_est = static_cast<unsigned>(off + nbytes);
+        off += Wb;
+        P->off_V = static_cast<unsigned>(off);
+        return off;
+    };
+    auto stripe = [&](size_t avail) {
+        return std::min(round_up(nr, 4), static_cast<int>(avail / row) & ~3);
+    };
+    for (size_t cap : {kTc2TwoCtas, smem_cap}) {
+        const int least = cap < smem_cap ? 8 : 16;  // rows of a stripe (and columns of a chunk)
+        size_t off = front(listed ? 0 : 1);
+        size_t num_end = listed ? P->off_est + nbytes : 0;
+        if (std::max(num_end, off + least * row + Eb) <= cap) {
+            P->VR = stripe(cap - off - Eb);
+            P->off_E = static_cast<unsigned>(off + P->VR * row);
             P->BC = cw;
             P->big = 0;
+            P->smem = std::max(num_end, off + P->VR * row + Eb);
             four_issuers(P);
             return true;
         }
-    }
-    // The chip operand in chunks of at most `avail` bytes: as few as fit, of even, equal widths.
-    auto chunk = [&](size_t avail) {
-        const int most = static_cast<int>(std::min<size_t>(cw, avail / P->PS)) & ~1;
-        if (most < 2) return 0;
-        const int n = (cw + most - 1) / most;
-        return std::min(most, round_up((cw + n - 1) / n, 2));
-    };
-    // Chunked layout: [W][P][S1][S2][red][zone], the zone holding T and V for the box sums,
-    // then the chunks of the chip operand, then num and the upper bounds.
-    {
-        size_t off = 0;
-        P->off_W = 0;
-        off += Wb;
-        P->off_P = static_cast<unsigned>(off);
-        off += Pb;
-        P->off_S1 = static_cast<unsigned>(off);
-        off += nbytes;
-        P->off_S2 = static_cast<unsigned>(off);
-        off += nbytes;
-        P->off_red = static_cast<unsigned>(off);
-        off += red;
-        off = a16(off);
-        const size_t zone_min = std::max(Tb + Vb, 2 * nbytes);
-        if (off + std::max(zone_min, 2 * static_cast<size_t>(P->PS)) <= smem_cap) {
-            const int bc = chunk(smem_cap - off);
-            if (bc < 2) return false;
-            P->BC = bc;
+        off = front(0);
+        num_end = listed ? P->off_est + nbytes : 0;
+        const size_t columns = std::min(cw, cap < smem_cap ? least : 2);
+        if (std::max(num_end, off + std::max(least * row, columns * P->PS)) <= cap) {
+            const int most = static_cast<int>(std::min<size_t>(cw, (cap - off) / P->PS)) & ~1;
+            const int n = (cw + most - 1) / most;
+            P->BC = std::min(most, round_up((cw + n - 1) / n, 2));
             P->big = 1;
-            P->off_E = P->off_T = P->off_num = static_cast<unsigned>(off);
-            P->off_V = static_cast<unsigned>(off + Tb);
-            P->off_est = static_cast<unsigned>(off + nbytes);
-            P->smem = off + std::max(zone_min, static_cast<size_t>(bc) * P->PS);
+            P->VR = stripe(cap - off);
+            P->off_E = P->off_V;
+            P->smem = std::max(num_end, off + std::max(P->VR * row, static_cast<size_t>(P->BC) * P->PS));
             four_issuers(P);
             return true;
         }
     }
-    // Striped layout (for geometries the others do not hold; the CUDA-core kernel took them at
-    // 73 ms over the chip-64 and chip-128, radius-48 passes of the batching configuration's 114 244
-    // points, this takes 5.8 ms): [S1][S2][red][P][W][zone], the zone holding V of a stripe of 16
-    // or more
-    // surface rows, then the chunks of the chip operand; num and the upper bounds take W and the
-    // zone once the products are done (P keeps its zero padding between points).
-    size_t off = 0;
-    P->off_S1 = 0;
-    off += nbytes;
-    P->off_S2 = static_cast<unsigned>(off);
-    off += nbytes;
-    P->off_red = static_cast<unsigned>(off);
-    off = a16(off + red);
-    P->off_P = static_cast<unsigned>(off);
-    off += Pb;
-    P->off_W = P->off_num = static_cast<unsigned>(off);
-    P->off_est = static_cast<unsigned>(off + nbytes);
-    const size_t num_end = off + 2 * nbytes;
-    off += Wb;
-    P->XV = round_up(cw + nc - 1, 4);
-    const size_t row = 2 * static_cast<size_t>(P->XV) * 4;
-    if (std::max(num_end, off + std::max<size_t>(16 * row, 2 * P->PS)) > smem_cap) return false;
-    const int bc = chunk(smem_cap - off);
-    if (bc < 2) return false;
-    P->BC = bc;
-    P->big = 2;
-    P->VR = std::min(round_up(nr, 16), static_cast<int>((smem_cap - off) / row) & ~15);
-    P->off_E = P->off_T = P->off_V = static_cast<unsigned>(off);
-    P->smem = std::max(num_end, off + std::max(P->VR * row, static_cast<size_t>(bc) * P->PS));
-    four_issuers(P);
-    return true;
+    return false;
 }
 
 template <typename T>
@@ -5447,7 +5251,6 @@ cudaError_t launch_track_impl(int dtype, const void* ref, const void* sec, const
         B.PS = TP.PS;
         B.PC = TP.PC;
         B.XS = TP.XS;
-        B.XT = TP.XT;
         B.NRS = TP.NRS;
         B.NRM = TP.NRM;
         B.NCM = TP.NCM;
@@ -5459,7 +5262,8 @@ cudaError_t launch_track_impl(int dtype, const void* ref, const void* sec, const
         B.MT = TP.MT;
         B.off_E = TP.off_E;
         B.off_W = TP.off_W;
-        B.off_T = TP.off_T;
+        B.off_R = TP.off_R;
+        B.roots = TP.roots;
         B.off_P = TP.off_P;
         B.off_V = TP.off_V;
         B.off_S1 = TP.off_S1;
