@@ -182,7 +182,7 @@ def profile_traffic(points, kernel):
 
 
 def fine_pass_kernel(ctx):
-    """The kernel the autotuner kept for the fine chip-32 / radius-25 pass (surface 50 x 50)."""
+    """The kernel of the fine chip-32 / radius-25 pass (surface 50 x 50)."""
     for t in ctx.tuned():
         if t["chip"] == [CHIP, CHIP] and t["surface"] == [2 * RADIUS, 2 * RADIUS]:
             return t["kernel"]
@@ -917,10 +917,8 @@ def gpu_arm(args):
     L = ar._lib
     ctx = L.Context(local)
     if args.profile:
-        # Under a profiler every launch is serialised and cold, which distorts the autotuner's
-        # timing of its samples (under ncu it kept k_corr_tc for the fine pass, which the
-        # timed run does not): profile runs take the fixed rule, which picks the kernels the
-        # tuned run keeps on this workload (k_corr_tc2 up to chip 64, k_corr_tc at chip 128).
+        # The kernels are the timed run's either way (k_corr_tc2 up to chip 64, k_corr_tc at chip
+        # 128); a profile run keeps no table of them.
         ctx.set_option(L.AR_OPT_AUTOTUNE, 0)
     a, b, valid, fdown = scene(ar, args.size, field=True)
     p = pipeline_params(ar, args.spacing if args.profile else SPACING)
