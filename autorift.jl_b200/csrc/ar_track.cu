@@ -4847,10 +4847,14 @@ void four_issuers(TcPlan* P) {
 // come first and the chip operand in chunks of BC columns in the stripe's place, without the
 // roots (they would cost a chip-64, radius-48 pass a chunk more). Either in half of an SM's
 // shared memory comes before either in all of it: 1.24 ms with two CTAs and chunks against 1.55
-// with one and the whole operand (14 400 points, chip 32, radius 44). The list of candidates of
+// with one and the whole operand (14 400 points, chip 32, radius 44). Not so for passes without a
+// point for each SM and one more (`many`), which wait for one point's latency (56 points at chip 16,
+// radius 40: 77 us a call with two, 75 with one), nor in chunks for surfaces up to 64 x 64, whose products
+// four threads issue where the SM is theirs alone (13 689 points at chip 128, radius 25: 3.93 ms
+// with two, 3.83 with one). The list of candidates of
 // surfaces up to 64 x 64 takes the place of W, V and E once the products are done (P keeps its
 // zero padding between points).
-bool plan_corr_tc(const PassGeometry& g, size_t smem_cap, TcPlan* P) {
+bool plan_corr_tc(const PassGeometry& g, size_t smem_cap, bool many, TcPlan* P) {
     const int ch = static_cast<int>(g.max_ch), cw = static_cast<int>(g.max_cw);
     const int nr = static_cast<int>(g.max_nr), nc = static_cast<int>(g.max_nc);
     if (nc > 128 || nr > 256 || nr < 1 || nc < 1 || cw < 2 || ch < 2 || (cw & 1)) return false;
@@ -4908,6 +4912,7 @@ bool plan_corr_tc(const PassGeometry& g, size_t smem_cap, TcPlan* P) {
         return std::min(round_up(nr, 4), static_cast<int>(avail / row) & ~3);
     };
     for (size_t cap : {kTc2TwoCtas, smem_cap}) {
+        if (cap < smem_cap && !many) continue;
         const int least = cap < smem_cap ? 8 : 16;  // rows of a stripe (and columns of a chunk)
         size_t off = front(listed ? 0 : 1);
         size_t num_end = listed ? P->off_est + nbytes : 0;
@@ -4920,6 +4925,7 @@ bool plan_corr_tc(const PassGeometry& g, size_t smem_cap, TcPlan* P) {
             four_issuers(P);
             return true;
         }
+        if (cap < smem_cap && listed) continue;
         off = front(0);
         num_end = listed ? P->off_est + nbytes : 0;
         const size_t columns = std::min(cw, cap < smem_cap ? least : 2);
@@ -5417,7 +5423,7 @@ cudaError_t launch_track_impl(int dtype, const void* ref, const void* sec, const
         // pass of radii 4 to 32 the two tie (73 523 points at chip 16: 3.9 ms).
         TcPlan TP2{}, TP1{};
         const bool fit2 = tc_ok && plan_corr_tc2(geom, 220 * 1024, &TP2);
-        const bool fit1 = tc_ok && plan_corr_tc(geom, 220 * 1024, &TP1);
+        const bool fit1 = tc_ok && plan_corr_tc(geom, 220 * 1024, pts.n > num_sms, &TP1);
         int kind = fit2 ? 2 : fit1 ? 1 : 0;
         const int force = scratch.uint8_kernel;
         if (force == 0 || (force == 1 && fit1) || (force == 2 && fit2)) kind = force;
