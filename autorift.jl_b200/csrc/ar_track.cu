@@ -2700,8 +2700,10 @@ __global__ void __launch_bounds__(kTc2Threads, 2) k_corr_tc2(const TcArgs A) {
             if (pow2) tc2_chip_stats(nnl, o.cs, o.c2, &mean, &sq);
             const double cnorm = __dsqrt_rn(sq);
             if (!__all_sync(kFull, tc::mbar_wait(&s_outb[b], ph, kTcWaitPolls))) {
-                // The main warps left, or will: wait for the barrier that ends them.
-                if (lane == 0) s_fail = 1;
+                // The main warps left, or are late: this point's output is lost, which the status
+                // says whatever they do. They are not told, as a flag set here could come
+                // between two main threads' reads of it: some would leave and the others wait for them.
+                if (lane == 0) atomicExch(A.status, 1);
                 __syncwarp();
                 ph ^= static_cast<uint32_t>(b);
                 continue;
@@ -2750,7 +2752,8 @@ __global__ void __launch_bounds__(kTc2Threads, 2) k_corr_tc2(const TcArgs A) {
     };
     for (int b = 0;; b ^= 1, ph ^= 1u) {
         // A wait that runs out leaves this thread with an empty point until the next barrier, where
-        // all of them leave.
+        // all of them leave. Only main threads write s_fail, before that barrier, and each reads it
+        // once after it and before another, so that they all see the same value.
         const bool got = tc::mbar_wait(&s_full, ph, kTcWaitPolls);
         if (!got) s_fail = 1;
         TC_PHASE(0)
