@@ -2532,6 +2532,7 @@ __global__ void __launch_bounds__(kTc2Threads, 2) k_corr_tc2(const TcArgs A) {
     __shared__ uint64_t s_mbar, s_full, s_free, s_outb[2];
     __shared__ uint32_t s_taddr;
     __shared__ int s_fail, s_more[2];  // s_more, by result slot: a measured point, or the end
+    __shared__ int s_lost;             // the patch warp gave up on a point
     __shared__ float s_bu;
     __shared__ float s_top[8], s_sec[8];
     __shared__ int s_at[8];
@@ -2572,7 +2573,7 @@ __global__ void __launch_bounds__(kTc2Threads, 2) k_corr_tc2(const TcArgs A) {
         tc::mbar_init(&s_outb[0], 8);
         tc::mbar_init(&s_outb[1], 8);
         tc::fence_mbar_init();
-        s_fail = 0;
+        s_fail = s_lost = 0;
     }
     if (tid < 4) s_isum[tid >> 1][tid & 1] = 0u;
     for (int e = tid; e < A.CWM * A.PC; e += kTc2Threads) s_P[e] = 0;
@@ -2701,9 +2702,9 @@ __global__ void __launch_bounds__(kTc2Threads, 2) k_corr_tc2(const TcArgs A) {
             const double cnorm = __dsqrt_rn(sq);
             if (!__all_sync(kFull, tc::mbar_wait(&s_outb[b], ph, kTcWaitPolls))) {
                 // The main warps left, or are late: this point's output is lost, which the status
-                // says whatever they do. They are not told, as a flag set here could come
+                // says in the end whatever they do. They are not told, as a flag set here could come
                 // between two main threads' reads of it: some would leave and the others wait for them.
-                if (lane == 0) atomicExch(A.status, 1);
+                if (lane == 0) s_lost = 1;
                 __syncwarp();
                 ph ^= static_cast<uint32_t>(b);
                 continue;
@@ -3444,6 +3445,7 @@ __global__ void __launch_bounds__(kTc2Threads, 2) k_corr_tc2(const TcArgs A) {
     }
     tc::fence_before_sync();
     __syncthreads();
+    if (tid == 0 && s_lost) atomicExch(A.status, 1);
     if (warp == 0) tc::tmem_dealloc(taddr, A.tmem_cols);
 }
 

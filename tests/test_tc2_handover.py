@@ -24,7 +24,7 @@ def explore(points, shared_flag):
     # Shared: phases completed of full, free, out[0], out[1] and the products; arrivals at out[*];
     # the points in the two slots; s_more; the flag; the status; outputs written.
     sh0 = dict(full=0, free=0, out=(0, 0), arr=(0, 0), issued=0, prods=0, pt=(None, None),
-               more=(1, 1), fail=0, status=0, written=0)
+               more=(1, 1), fail=0, lost=0, status=0, written=0)
     main0 = dict(pc="full", b=0, ph=0, mb=0, got=0, ok=1, failed=0, phase=0)
     local0 = (dict(main0), dict(main0), dict(pc="bar", b=0, ph=0, then="more"),
               dict(pc="fetch", b=0, ph=0, n=0))
@@ -95,7 +95,7 @@ def explore(points, shared_flag):
                 return [(sh, dict(me, pc="gave up"))]  # its store comes any time later
             if pc == "gave up":
                 nxt = dict(me, b=me["b"] ^ 1, ph=me["ph"] ^ me["b"], pc="bar")
-                return [(dict(sh, fail=1) if shared_flag else dict(sh, status=1), nxt)]
+                return [(dict(sh, **{"fail" if shared_flag else "lost": 1}), nxt)]
             return None
         if pc == "fetch":
             sh["pt"] = put(sh["pt"], me["b"], me["n"] if me["n"] < points else -1)
@@ -142,7 +142,7 @@ def explore(points, shared_flag):
                     l2[i] = m
                 nxt.append((dict(sh), tuple(l2)))
         if all(m["pc"] == "gone" for m in ls):
-            finals.append(sh)
+            finals.append(dict(sh, status=sh["status"] | sh["lost"]))  # thread 0, after the last barrier
         elif not nxt:
             raise AssertionError("deadlock: " + ", ".join(m["pc"] for m in ls))
         stack.extend(nxt)
@@ -163,12 +163,16 @@ def test_the_model_finds_the_shared_flags_fault():
 
 
 def test_kernel_follows_the_model():
-    """The patch warp reports a wait that ran out to the status word itself; only main warps touch
-    the flag that makes the main warps leave."""
+    """The patch warp keeps a wait that ran out in a word of its own, which reaches the status after the
+    barrier that ends the block; only main warps touch the flag that makes the main warps leave."""
     text = SRC.read_text()
     body = text[text.index("k_corr_tc2(const TcArgs A) {"):]
+    body = re.sub(r"// [A-Za-z][^\n]*", "", body[:body.index("__global__")])
     patch = body[body.index("} else if (warp == 9) {"):]
-    patch = re.sub(r"//[^\n]*", "", patch[:patch.index("// ---", 200)])
+    patch = patch[:patch.index("// ---", 200)]
     assert "s_fail" not in patch
     gave_up = patch[patch.index("if (!__all_sync(kFull, tc::mbar_wait(&s_outb[b]"):]
-    assert "atomicExch(A.status, 1)" in gave_up[:gave_up.index("continue;")]
+    assert "s_lost = 1" in gave_up[:gave_up.index("continue;")]
+    assert body.count("s_lost") == 4
+    last = body.rindex("__syncthreads();")
+    assert "if (tid == 0 && s_lost) atomicExch(A.status, 1);" in body[last:]
