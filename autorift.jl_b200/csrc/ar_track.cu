@@ -1788,8 +1788,6 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_corr_tc(const TcArgs A) {
             continue;  // degenerate chip: searched, no measurement (src/track.jl:286)
         TC_PHASE(3)
         const double cnorm = __dsqrt_rn(sq);
-        // The point is measured: its refinement slot is taken now, read after later barriers.
-        if (tid == 0 && !(A.up == 1 || nr < 5 || nc < 5)) s_slot = atomicAdd(A.sub_count, 1);
         const double nn = static_cast<double>(nnl);
 
         // Box sums carried from the held point: same window columns and shape, `sh` rows
@@ -1986,7 +1984,8 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_corr_tc(const TcArgs A) {
                 // The previous chunk's products must be done before its rows are replaced.
                 ok = tc::mbar_wait(&s_mbar, phase, kTcWaitPolls);
                 phase ^= 1u;
-                if (__syncthreads_or(!ok)) break;
+                ok = !__syncthreads_or(!ok);
+                if (!ok) break;
                 tc::fence_after_sync();
             }
             // E: NB rows u = 16 - NB ... 15 per chip column, row u at e = u - 16 + NB: 16 bytes
@@ -2090,6 +2089,9 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_corr_tc(const TcArgs A) {
         // The peak or its 5 x 5 patch (all inside the surface): the numerators of the output.
         const bool single = A.up == 1 || nr < 5 || nc < 5;
         const int span = single ? 1 : 5;
+        // The products are here and nothing below gives up, so the patch of this slot of the
+        // refinement queue will be written (k_refine trusts the count). Read after later barriers.
+        if (tid == 0 && !single) s_slot = atomicAdd(A.sub_count, 1);
         int pi0 = 0, pj0 = 0;
         auto patch_at = [&](int i, int j) {
             pi = i;
@@ -3712,7 +3714,6 @@ __global__ void __launch_bounds__(kBfThreads, 1) k_corr_bf(const BfArgs A) {
         const double cnorm = __dsqrt_rn(sq);
         const double cshift = Tr::integer ? rint(mean) : static_cast<double>(__double2float_rn(mean));
         const float csf = static_cast<float>(cshift);
-        if (tid == 0 && !(A.up == 1 || nr < 5 || nc < 5)) s_slot = atomicAdd(A.sub_count, 1);
         TC_PHASE(2)
 
         // Box sums in FP64, a stripe of window columns at a time: the stripe's image values
@@ -4042,6 +4043,9 @@ __global__ void __launch_bounds__(kBfThreads, 1) k_corr_bf(const BfArgs A) {
             failed = true;
             break;
         }
+        // The products are here and nothing below gives up, so the patch of this slot of the
+        // refinement queue will be written (k_refine trusts the count).
+        if (tid == 0 && !(A.up == 1 || nr < 5 || nc < 5)) s_slot = atomicAdd(A.sub_count, 1);
 
         // Epilogue: every value normalised in FP64 into the surface in shared memory.
         {
