@@ -217,6 +217,7 @@ struct CorrArgs {
     float* surf_out;  // optional: each point's surface, NRS x NCM floats per point
     unsigned long long* flops;  // optional: algorithmic FLOPs of the surfaces computed
     unsigned off_surf2;  // rotation search: the best surface so far (NRS x NCM floats)
+    int GTI, GTJ;        // k_corr_fp, Float32: the surface tile k_corr would take
     Rotation rot;        // rotation search angles (k_corr<T, true> only)
 };
 static_assert(sizeof(CorrArgs) <= 4096, "k_corr's arguments must fit the 4 KB parameter space");
@@ -722,6 +723,46 @@ __device__ __noinline__ float fp_exact(double num, double wvar, double cnorm) {
     return den > 0.0 ? __double2float_rn(__ddiv_rn(num, den)) : 0.0f;
 }
 
+// The variance terms that NaN and infinite pixels of a Float32 window reach, as in k_corr's tables: an
+// FP64 sum that took in a NaN, or let an infinity go, is a NaN from there on. So such a pixel reaches
+// every later row of its tile and every later column of its run of sixteen, and a variance that is
+// not a number counts as none (the value is 0). The other terms were summed with these pixels as zero.
+// `first` holds two rows a window column: the first with a NaN, the first with an infinity. Against
+// such windows left to sums that start afresh more often (other peaks than k_corr's beside a gap), this
+// costs windows without gaps 0.3 % at chip 32, radius 25 and 1.5 % at chip 16, radius 10 (the second copy of
+// the sums in the kernel; out of line 0.1 and 0.8 %, but 6 % behind k_corr over gaps).
+__device__ __noinline__ void fp_nonfinite(const float2* win, int XH, int WS, int ch, int cw, int nr, int nc,
+                                          int TI, int TJ, bool ncc, double* wv, int NRS, int* first) {
+    const int tid = threadIdx.x;  // at least as many as window columns
+    const float2* col = win + ((tid & 1) * XH + (tid >> 1)) * WS;
+    for (int ti = 0; ti < nr; ti += TI) {
+        const int te = min(ti + TI, nr), none = te + ch;
+        if (tid < cw + nc - 1) {
+            int rn = none, ri = none;
+            for (int r = ti; r < te + ch - 1 && rn == none; ++r) {
+                const float v = fabsf(col[r].x);
+                if (isnan(v)) rn = r;
+                else if (!(v <= FLT_MAX)) ri = min(ri, r);
+            }
+            first[2 * tid] = rn;
+            first[2 * tid + 1] = ri;
+        }
+        __syncthreads();
+        if (tid < nc) {
+            const int run = tid - ((tid % TJ) & 15);  // the sums along a row start afresh here
+            int rn = none, ri = none;
+            for (int x = run; x < tid + cw; ++x) {
+                rn = min(rn, x < tid ? min(first[2 * x], first[2 * x + 1]) : first[2 * x]);
+                if (x >= tid) ri = min(ri, first[2 * x + 1]);
+            }
+            const int rb = min(rn, ri);
+            for (int i = max(ti, rb - ch + 1); i < te; ++i)
+                wv[tid * NRS + i] = ncc && i <= rb && i + ch <= rn ? INFINITY : 0.0;
+        }
+        __syncthreads();
+    }
+}
+
 template <typename T, bool ROT>
 __global__ void __launch_bounds__(kCorrThreads, 2) k_corr_fp(const CorrArgs A) {
     typedef Traits<T> Tr;
@@ -974,7 +1015,10 @@ __global__ void __launch_bounds__(kCorrThreads, 2) k_corr_fp(const CorrArgs A) {
             // surface rows; A.TI rows of each segment at a time go to shared memory, where a task
             // sums cw columns for five neighbouring values. The counts of non-zero values keep
             // windows of zeros at exactly zero, which sliding FP64 sums would miss by a rounding.
-            if (!have_var) {
+            // kGaps: a Float32 window with pixels that are not finite, which count as zero.
+            bool nonfinite = false;  // a column sum of this thread took one in
+            auto box_sums = [&](auto gaps) {
+                constexpr bool kGaps = decltype(gaps)::value;
                 const int nseg = max(1, min(8, kCorrThreads / XW));
                 const int seglen = (nr + nseg - 1) / nseg;
                 const int seg = tid / XW, x = tid - seg * XW;
@@ -987,6 +1031,7 @@ __global__ void __launch_bounds__(kCorrThreads, 2) k_corr_fp(const CorrArgs A) {
                     if constexpr (Tr::integer) {
                         return static_cast<BS>(__float_as_int(__fadd_rn(__fadd_rn(v, cs), 12582912.0f)) - 0x4B400000);
                     } else {
+                        if (kGaps && !(fabsf(v) <= FLT_MAX)) return 0.0;
                         return __dadd_rn(static_cast<double>(v), cshift);
                     }
                 };
@@ -1097,6 +1142,18 @@ __global__ void __launch_bounds__(kCorrThreads, 2) k_corr_fp(const CorrArgs A) {
                         }
                     }
                     __syncthreads();
+                }
+                // From a pixel that is not finite on, its column's sums are not either.
+                if constexpr (!Tr::integer && !kGaps) nonfinite = !(h2 <= DBL_MAX);
+            };
+            if (!have_var) {
+                box_sums(std::false_type{});
+                if constexpr (!Tr::integer) {
+                    if (__syncthreads_or(nonfinite)) {
+                        box_sums(std::true_type{});
+                        fp_nonfinite(s_win, XH, A.WS, ch, cw, nr, nc, A.GTI, A.GTJ, A.measure == AR_NCC, s_wv,
+                                     A.NRS, reinterpret_cast<int*>(s_v1));
+                    }
                 }
                 have_var = Tr::integer;  // Float32 image values carry the shift's rounding
             }
@@ -5217,6 +5274,12 @@ cudaError_t launch_track_impl(int dtype, const void* ref, const void* sec, const
     A.measure = measure;
     A.TI = P.TI;
     A.TJ = P.TJ;
+    if (fp && dtype == AR_F32) {
+        CorrPlan G{};
+        const bool fits = plan_corr(geom, ph_bytes, 220 * 1024, &G, rotating);
+        A.GTI = fits ? G.TI : P.NRS;
+        A.GTJ = fits ? G.TJ : P.NCM;
+    }
     A.CHP = P.CHP;
     A.CWM = P.CWM;
     A.BC = P.BC;
