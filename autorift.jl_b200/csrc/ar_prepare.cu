@@ -4,7 +4,7 @@
 //
 // Stencils. The mask-aware box mean (src/preprocess.jl:371-399 over src/window.jl:228-439)
 // is a shared-memory tile: per-pixel values and "contributes" flags (valid and not NaN) for a
-// 32x64 output tile plus its halo, FP64 column sums, then FP64 row sums, divided by the count
+// 32x64 (narrow windows: 32x32) output tile plus its halo, FP64 column sums, then FP64 row sums, divided by the count
 // and rounded to Float32. For integer images and for Float32 images of bounded dynamic range
 // every partial sum is an exact FP64 value, so the mean equals the reference's banded running
 // sum bit for bit. Erosion of the validity mask (src/preprocess.jl:447-460) is the same
@@ -30,10 +30,8 @@ namespace ar {
 namespace {
 
 constexpr int kTile = 32;      // output rows of a box tile: a lane each
-constexpr int kTileC = 64;     // output columns
-constexpr int kRun = 8;        // consecutive window sums a thread makes at a time
 constexpr int kBoxThreads = 256;
-static_assert(kTile * (kTileC / kRun) == kBoxThreads, "one run of columns per thread");
+constexpr int kSms = 148;      // of the GPU this is written for
 constexpr int kMaxWidth = 63;
 constexpr int kStatBlocks = 592;
 constexpr int kStatThreads = 256;
@@ -47,12 +45,28 @@ __device__ __forceinline__ float as_f32(T v) {
 // Which per-pixel quantity a box pass averages.
 enum BoxMode { BOX_IMAGE = 0, BOX_DEV2 = 1 };
 
+// The two tile shapes. Windows below eight share too little in runs of eight, and leave most of a
+// 64-column tile's loads to a nearly empty second round: highpass of a 2001 x 1503 Float32 image at width 3, 5
+// and 7 took 35, 40 and 47 us with a fresh sum a window, 43, 45 and 50 in wide tiles, and takes 33, 35 and 37
+// in narrow ones. From eight on wide tiles are ahead (the two Wallis passes at width 9, 21: 75 and 90 against
+// 79 and 109 us), except where narrow ones do not fill the SMs twice and a tile's latency is what counts
+// (512 x 512, highpass at width 9, 21: 11 and 13 us wide, 7 and 10 narrow).
+template <int COLS, int RUN, int LOADS>
+struct BoxShape {
+    static constexpr int kCols = COLS;    // output columns of a tile
+    static constexpr int kRun = RUN;      // consecutive window sums a thread makes at a time
+    static constexpr int kLoads = LOADS;  // columns a warp loads at a time
+    static_assert(kTile * (COLS / RUN) == kBoxThreads, "one run of columns per thread");
+};
+typedef BoxShape<64, 8, 4> BoxWide;
+typedef BoxShape<32, 4, 5> BoxNarrow;
+
 // Shared-memory layout of one tile with its halo: values, flags, column sums. The window is
 // (wx, wy) after the reference's clamp to the image (src/window.jl:632-637), with the extra
 // element of an even width on the left (src/window.jl:254-257). Column strides are odd, so that
 // lanes on consecutive columns hit different banks.
 struct BoxSmem {
-    float* val;       // Rr x Rc, Rr = kTile + wy - 1, Rc = kTileC + wx - 1, column-major, stride Rr | 1
+    float* val;       // Rr x Rc, Rr = kTile + wy - 1, Rc = kCols + wx - 1, column-major, stride Rr | 1
     uint8_t* flag;    // the same: 1 contributes to the mean, 2 in the image and invalid
     double* vs;       // kTile x Rc column sums, stride kTile + 1
     uint32_t* vf;     // the same: contributing count, invalid count << 16
@@ -70,12 +84,12 @@ __device__ __forceinline__ float dev2_of(float x, bool m, float mean, bool* cont
     return 0.0f;
 }
 
-// Eight consecutive window sums of length w over x(0), x(1), ..., out(k, sum of x(k) .. x(k + w - 1)).
+// kRun consecutive window sums of length w over x(0), x(1), ..., out(k, sum of x(k) .. x(k + w - 1)).
 // No value is ever subtracted, so a value that leaves the window leaves no rounding (nor an
 // infinity) behind. From w = kRun on, a window is the tail of the run's first kRun values, the
 // values common to the run, and the head of the kRun - 1 that follow: w + 2 kRun additions for
 // the run instead of w kRun.
-template <typename Get, typename Out>
+template <int kRun, typename Get, typename Out>
 __device__ __forceinline__ void run_sums(int w, Get x, Out out) {
     if (w >= kRun) {
         double tail[kRun], v[kRun];
@@ -93,6 +107,13 @@ __device__ __forceinline__ void run_sums(int w, Get x, Out out) {
             mid = __dadd_rn(mid, v[k]);
             out(k, __dadd_rn(tail[k], mid));
         }
+    } else if constexpr (kRun == 4) {
+        double v[kRun + 2];  // at most three values a window
+#pragma unroll
+        for (int k = 0; k < kRun + 2; ++k) v[k] = k < kRun + w - 1 ? x(k) : 0.0;
+#pragma unroll
+        for (int k = 0; k < kRun; ++k)
+            out(k, __dadd_rn(__dadd_rn(__dadd_rn(0.0, v[k]), w > 1 ? v[k + 1] : 0.0), w > 2 ? v[k + 2] : 0.0));
     } else {
 #pragma unroll
         for (int k = 0; k < kRun; ++k) {
@@ -107,23 +128,25 @@ __device__ __forceinline__ void run_sums(int w, Get x, Out out) {
 // contributing neighbours and whether every in-bounds neighbour is valid.
 //   Bound: shared-memory reads and FP64 additions per pixel. With fresh sums of every window (w reads
 // and additions a direction) the two Wallis passes of a 3000 x 3000 Float32 image at width 21 took
-// 225 and 306 us; in runs of eight, with loads that do not wait on a bounds check, 96 and 130.
-template <typename T, int MODE, typename Out>
+// 225 and 306 us; in runs (BoxShape), with loads that do not wait on a bounds check, 96 and 130.
+template <typename T, int MODE, typename Shape, typename Out>
 __device__ void box_tile(const T* img, const uint8_t* mask, const float* mean, int64_t nr,
                          int64_t nc, int wx, int wy, int64_t r0, int64_t c0, BoxSmem S, Out out) {
     const int ly = wy / 2, lx = wx / 2;
-    const int Rr = kTile + wy - 1, Rc = kTileC + wx - 1, ld = Rr | 1;
-    constexpr int ldv = kTile + 1;
+    const int Rr = kTile + wy - 1, Rc = Shape::kCols + wx - 1, ld = Rr | 1;
+    constexpr int ldv = kTile + 1, kRun = Shape::kRun;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // Warps over columns (four at a time, so that their loads are in flight together), lanes over
-    // rows, from addresses that are always valid.
-    for (int cb = 4 * warp; cb < Rc; cb += 4 * (kBoxThreads / 32))
+    // Warps over columns (kLoads at a time, so that their loads are in flight together; in narrow
+    // tiles eight warps then take all of them at once), lanes over rows, from addresses that are always
+    // valid.
+    constexpr int kLoads = Shape::kLoads;
+    for (int cb = kLoads * warp; cb < Rc; cb += kLoads * (kBoxThreads / 32))
         for (int r = lane; r < Rr; r += 32) {
-            float x[4], mn[4];
-            uint8_t mk[4];
+            float x[kLoads], mn[kLoads];
+            uint8_t mk[kLoads];
             const int64_t gr = r0 - ly + r, grc = min(max(gr, static_cast<int64_t>(0)), nr - 1);
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < kLoads; ++u) {
                 const int64_t gc = c0 - lx + cb + u;
                 const int64_t g = grc + min(max(gc, static_cast<int64_t>(0)), nc - 1) * nr;
                 x[u] = as_f32(img[g]);
@@ -131,7 +154,7 @@ __device__ void box_tile(const T* img, const uint8_t* mask, const float* mean, i
                 mn[u] = MODE == BOX_IMAGE ? 0.0f : mean[g];
             }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < kLoads; ++u) {
                 if (cb + u >= Rc) continue;
                 const int64_t gc = c0 - lx + cb + u;
                 const bool in = gr == grc && gc >= 0 && gc < nc, m = mk[u] != 0;
@@ -154,7 +177,7 @@ __device__ void box_tile(const T* img, const uint8_t* mask, const float* mean, i
         const float* v = S.val + c * ld + i0;
         const uint8_t* f = S.flag + c * ld + i0;
         double* vs = S.vs + c * ldv + i0;
-        run_sums(wy, [&](int k) { return static_cast<double>(v[k]); }, [&](int k, double s) { vs[k] = s; });
+        run_sums<kRun>(wy, [&](int k) { return static_cast<double>(v[k]); }, [&](int k, double s) { vs[k] = s; });
         auto word = [&](int k) { return static_cast<uint32_t>(f[k] & 1) | (static_cast<uint32_t>(f[k] & 2) << 15); };
         uint32_t n = 0u;
         for (int k = 0; k < wy; ++k) n += word(k);
@@ -173,7 +196,7 @@ __device__ void box_tile(const T* img, const uint8_t* mask, const float* mean, i
         const int64_t gr = r0 + lane;
         uint32_t n = 0u;
         for (int k = 0; k < wx; ++k) n += vf[k * ldv];
-        run_sums(wx, [&](int k) { return vs[k * ldv]; }, [&](int k, double s) {
+        run_sums<kRun>(wx, [&](int k) { return vs[k * ldv]; }, [&](int k, double s) {
             if (gr < nr && c0 + j0 + k < nc) out(gr + (c0 + j0 + k) * nr, s, static_cast<int>(n & 0xFFFFu), (n >> 16) == 0u);
             if (k + 1 < kRun) n += vf[(k + wx) * ldv] - vf[k * ldv];
         });
@@ -200,8 +223,9 @@ struct BoxDiv {
     }
 };
 
+template <typename Shape>
 __device__ BoxSmem box_smem(unsigned char* base, int wx, int wy) {
-    const int ld = (kTile + wy - 1) | 1, Rc = kTileC + wx - 1;
+    const int ld = (kTile + wy - 1) | 1, Rc = Shape::kCols + wx - 1;
     BoxSmem S;
     size_t off = 0;
     S.vs = reinterpret_cast<double*>(base + off);
@@ -214,25 +238,26 @@ __device__ BoxSmem box_smem(unsigned char* base, int wx, int wy) {
     return S;
 }
 
+template <typename Shape>
 constexpr size_t box_smem_bytes(int wx, int wy) {
-    const size_t ld = (kTile + wy - 1) | 1, Rc = kTileC + wx - 1;
+    const size_t ld = (kTile + wy - 1) | 1, Rc = Shape::kCols + wx - 1;
     return (sizeof(double) + sizeof(uint32_t)) * (kTile + 1) * Rc + (sizeof(float) + 1) * ld * Rc + 64;
 }
-static_assert(box_smem_bytes(kMaxWidth, kMaxWidth) <= static_cast<size_t>(kDynSmemCap),
+static_assert(box_smem_bytes<BoxWide>(kMaxWidth, kMaxWidth) <= static_cast<size_t>(kDynSmemCap),
               "every accepted window fits");
 
 // Highpass (src/preprocess.jl:304-312) with `_filtered`: out = img - boxmean where valid,
 // zero and invalid elsewhere; the mask erodes by the filter width.
-template <typename T>
+template <typename T, typename Shape>
 __global__ void __launch_bounds__(kBoxThreads) k_highpass(const T* img, const uint8_t* mask,
                                                           int64_t nr, int64_t nc, int wx, int wy,
                                                           float* out, uint8_t* vout) {
     extern __shared__ __align__(16) unsigned char bsm[];
-    const BoxSmem S = box_smem(bsm, wx, wy);
+    const BoxSmem S = box_smem<Shape>(bsm, wx, wy);
     const BoxDiv div(wx, wy);
     const int64_t r0 = static_cast<int64_t>(blockIdx.x) * kTile;
-    const int64_t c0 = static_cast<int64_t>(blockIdx.y) * kTileC;
-    box_tile<T, BOX_IMAGE>(img, mask, nullptr, nr, nc, wx, wy, r0, c0, S,
+    const int64_t c0 = static_cast<int64_t>(blockIdx.y) * Shape::kCols;
+    box_tile<T, BOX_IMAGE, Shape>(img, mask, nullptr, nr, nc, wx, wy, r0, c0, S,
                            [&](int64_t g, double s, int cnt, bool eroded) {
                                const float mean = div.mean(s, cnt);
                                float o = (mask[g] && isfinite(mean)) ? __fsub_rn(as_f32(img[g]), mean)
@@ -540,31 +565,31 @@ size_t highpass_int_smem(int wx, int wy, int TR) {
 }
 
 // First Wallis pass: the masked box mean (src/preprocess.jl:336).
-template <typename T>
+template <typename T, typename Shape>
 __global__ void __launch_bounds__(kBoxThreads) k_boxmean(const T* img, const uint8_t* mask,
                                                          int64_t nr, int64_t nc, int wx, int wy,
                                                          float* mean) {
     extern __shared__ __align__(16) unsigned char bsm[];
-    const BoxSmem S = box_smem(bsm, wx, wy);
+    const BoxSmem S = box_smem<Shape>(bsm, wx, wy);
     const BoxDiv div(wx, wy);
     const int64_t r0 = static_cast<int64_t>(blockIdx.x) * kTile;
-    const int64_t c0 = static_cast<int64_t>(blockIdx.y) * kTileC;
-    box_tile<T, BOX_IMAGE>(img, mask, nullptr, nr, nc, wx, wy, r0, c0, S,
+    const int64_t c0 = static_cast<int64_t>(blockIdx.y) * Shape::kCols;
+    box_tile<T, BOX_IMAGE, Shape>(img, mask, nullptr, nr, nc, wx, wy, r0, c0, S,
                            [&](int64_t g, double s, int cnt, bool) { mean[g] = div.mean(s, cnt); });
 }
 
 // Second Wallis pass (src/preprocess.jl:337-351, 416-438) with `_filtered`.
-template <typename T>
+template <typename T, typename Shape>
 __global__ void __launch_bounds__(kBoxThreads) k_wallis(const T* img, const uint8_t* mask,
                                                         const float* mean, int64_t nr,
                                                         int64_t nc, int wx, int wy, float floor_sd,
                                                         float* out, uint8_t* vout) {
     extern __shared__ __align__(16) unsigned char bsm[];
-    const BoxSmem S = box_smem(bsm, wx, wy);
+    const BoxSmem S = box_smem<Shape>(bsm, wx, wy);
     const BoxDiv div(wx, wy);
     const int64_t r0 = static_cast<int64_t>(blockIdx.x) * kTile;
-    const int64_t c0 = static_cast<int64_t>(blockIdx.y) * kTileC;
-    box_tile<T, BOX_DEV2>(img, mask, mean, nr, nc, wx, wy, r0, c0, S,
+    const int64_t c0 = static_cast<int64_t>(blockIdx.y) * Shape::kCols;
+    box_tile<T, BOX_DEV2, Shape>(img, mask, mean, nr, nc, wx, wy, r0, c0, S,
                           [&](int64_t g, double s, int cnt, bool eroded) {
                               float msd = div.mean(s, cnt);
                               // sqrt(max(msd, 0f0)): Julia's max keeps a NaN.
@@ -850,26 +875,26 @@ cudaError_t quantize_u8(const T* img, const uint8_t* mask, int64_t n, QuantStats
 }
 
 // The box-tile filters: highpass of float imagery, and Wallis.
-template <typename T>
+template <typename T, typename Shape>
 cudaError_t launch_box(const PrepareJob& J, const T* img, int wx, int wy, float* filt, cudaStream_t s) {
     const dim3 grid(static_cast<unsigned>((J.nrows + kTile - 1) / kTile),
-                    static_cast<unsigned>((J.ncols + kTileC - 1) / kTileC));
-    const size_t smem = box_smem_bytes(wx, wy);
+                    static_cast<unsigned>((J.ncols + Shape::kCols - 1) / Shape::kCols));
+    const size_t smem = box_smem_bytes<Shape>(wx, wy);
     auto cap = [](auto* kernel) {
         return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDynSmemCap);
     };
     cudaError_t e;
     if (J.preprocess == 1) {
-        e = cap(k_highpass<T>);
+        e = cap(k_highpass<T, Shape>);
         if (e != cudaSuccess) return e;
-        k_highpass<T><<<grid, kBoxThreads, smem, s>>>(img, J.mask, J.nrows, J.ncols, wx, wy, filt, J.vout);
+        k_highpass<T, Shape><<<grid, kBoxThreads, smem, s>>>(img, J.mask, J.nrows, J.ncols, wx, wy, filt, J.vout);
     } else {
-        e = cap(k_boxmean<T>);
-        if (e == cudaSuccess) e = cap(k_wallis<T>);
+        e = cap(k_boxmean<T, Shape>);
+        if (e == cudaSuccess) e = cap(k_wallis<T, Shape>);
         if (e != cudaSuccess) return e;
-        k_boxmean<T><<<grid, kBoxThreads, smem, s>>>(img, J.mask, J.nrows, J.ncols, wx, wy, J.mtmp);
-        k_wallis<T><<<grid, kBoxThreads, smem, s>>>(img, J.mask, J.mtmp, J.nrows, J.ncols, wx, wy,
-                                                        static_cast<float>(J.min_std), filt, J.vout);
+        k_boxmean<T, Shape><<<grid, kBoxThreads, smem, s>>>(img, J.mask, J.nrows, J.ncols, wx, wy, J.mtmp);
+        k_wallis<T, Shape><<<grid, kBoxThreads, smem, s>>>(img, J.mask, J.mtmp, J.nrows, J.ncols, wx, wy,
+                                                               static_cast<float>(J.min_std), filt, J.vout);
     }
     return cudaSuccess;
 }
@@ -924,7 +949,9 @@ cudaError_t prepare_t(const PrepareJob& J, cudaStream_t s, long long* launches) 
                                                          filt, J.vout);
         *launches += 1;
     } else {
-        e = launch_box<T>(J, img, wx, wy, filt, s);
+        const int64_t narrow = (J.nrows + kTile - 1) / kTile * ((J.ncols + BoxNarrow::kCols - 1) / BoxNarrow::kCols);
+        e = std::max(wx, wy) < BoxWide::kRun || narrow <= 2 * kSms ? launch_box<T, BoxNarrow>(J, img, wx, wy, filt, s)
+                                                                   : launch_box<T, BoxWide>(J, img, wx, wy, filt, s);
         if (e != cudaSuccess) return e;
         *launches += J.preprocess == 1 ? 1 : 2;
     }
