@@ -459,10 +459,12 @@ __global__ void __launch_bounds__(kCorrThreads, 2) k_corr(const CorrArgs A) {
                             const int r = task % wrows, seg = task / wrows;
                             const int j0s = seg << 4, j1s = min(j0s + 16, tcols);
                             PH h1 = 0, h2 = 0;
+                            int nz = 0;  // Float32: values other than zero
                             for (int b = 0; b < bc; ++b) {
                                 const PH w = wv((j0s + b) * A.WS + r);
                                 h1 = h1 + w;
                                 h2 = h2 + w * w;
+                                if (!Tr::integer) nz += w != PH(0);
                             }
                             for (int jj = j0s; jj < j1s; ++jj) {
                                 if (jj > j0s) {
@@ -470,7 +472,11 @@ __global__ void __launch_bounds__(kCorrThreads, 2) k_corr(const CorrArgs A) {
                                     const PH wn = wv((jj - 1 + bc) * A.WS + r);
                                     h1 = h1 + wn - wo;
                                     h2 = h2 + wn * wn - wo * wo;
+                                    if (!Tr::integer) nz += (wn != PH(0)) - (wo != PH(0));
                                 }
+                                // A row of zeros sums to zero: sliding FP64 sums of Float32 values may
+                                // miss it by a rounding, which would stand for a variance.
+                                if (!Tr::integer && nz == 0 && h2 == h2) h1 = h2 = PH(0);
                                 PH* p1 = &s_ph1[jj * A.PHS + r + 1];
                                 PH* p2 = &s_ph2[jj * A.PHS + r + 1];
                                 *p1 = b0 == 0 ? h1 : *p1 + h1;
@@ -513,7 +519,22 @@ __global__ void __launch_bounds__(kCorrThreads, 2) k_corr(const CorrArgs A) {
                         }
                     }
                     __syncthreads();
-                    // Exclusive prefix down each column by warp scans: ph[jl][q] = sum_{r<q} H[r].
+                    // Exclusive prefix down each column: ph[jl][q] = sum_{r<q} H[r]. Float32: in row
+                    // order, a thread a column, so that rows of zeros leave it as it was and windows of
+                    // zeros keep exactly zero variance (a scan adds each row's sum in an order of its
+                    // own). Integer types (exact sums): by warp scans.
+                    if constexpr (!Tr::integer) {
+                        for (int jw = tid; jw < tcols; jw += bd) {
+                            PH* p1 = s_ph1 + jw * A.PHS;
+                            PH* p2 = s_ph2 + jw * A.PHS;
+                            PH c1 = 0, c2 = 0;
+                            p1[0] = p2[0] = PH(0);
+                            for (int q = 1; q <= wrows; ++q) {
+                                p1[q] = c1 = c1 + p1[q];
+                                p2[q] = c2 = c2 + p2[q];
+                            }
+                        }
+                    } else
                     for (int jw = warp; jw < tcols; jw += nwarps) {
                         PH c1 = 0, c2 = 0;
                         for (int q = 1; q <= wrows; q += 32) {
