@@ -520,19 +520,22 @@ __global__ void __launch_bounds__(kCorrThreads, 2) k_corr(const CorrArgs A) {
                     }
                     __syncthreads();
                     // Exclusive prefix down each column: ph[jl][q] = sum_{r<q} H[r]. Float32: in row
-                    // order, a thread a column, so that rows of zeros leave it as it was and windows of
-                    // zeros keep exactly zero variance (a scan adds each row's sum in an order of its
-                    // own). Integer types (exact sums): by warp scans.
+                    // order, a thread a column and table, so that rows of zeros leave it as it was and
+                    // windows of zeros keep exactly zero variance (a scan adds each row's sum in an
+                    // order of its own). Integer types (exact sums): by warp scans.
                     if constexpr (!Tr::integer) {
-                        for (int jw = tid; jw < tcols; jw += bd) {
-                            PH* p1 = s_ph1 + jw * A.PHS;
-                            PH* p2 = s_ph2 + jw * A.PHS;
-                            PH c1 = 0, c2 = 0;
-                            p1[0] = p2[0] = PH(0);
-                            for (int q = 1; q <= wrows; ++q) {
-                                p1[q] = c1 = c1 + p1[q];
-                                p2[q] = c2 = c2 + p2[q];
+                        for (int t = tid; t < 2 * tcols; t += bd) {
+                            PH* p = t < tcols ? s_ph1 + t * A.PHS : s_ph2 + (t - tcols) * A.PHS;
+                            PH c = 0, v[4];  // four rows loaded ahead of their sums' stores
+                            p[0] = PH(0);
+                            int q = 1;
+                            for (; q + 3 <= wrows; q += 4) {
+    #pragma unroll
+                                for (int u = 0; u < 4; ++u) v[u] = p[q + u];
+    #pragma unroll
+                                for (int u = 0; u < 4; ++u) p[q + u] = c = c + v[u];
                             }
+                            for (; q <= wrows; ++q) p[q] = c = c + p[q];
                         }
                     } else
                     for (int jw = warp; jw < tcols; jw += nwarps) {
