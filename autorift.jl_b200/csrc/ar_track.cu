@@ -4704,6 +4704,19 @@ bool plan_corr_fp(const PassGeometry& g, size_t smem_cap, bool rot, bool integer
     return off <= smem_cap;
 }
 
+// Whether k_corr_fp is the faster kernel of a one-tile surface. What it saves grows with the chip
+// and the surface, while its barriers and half-filled steps around the products do not shrink with them.
+// k_corr's time over k_corr_fp's on some 4000 points, without refinement: Float32 and UInt16 chip 4 radius 6
+// 0.88, chip 8 radius 12 0.95 and 16 1.15, chip 12 radius 10 0.97 and 16 1.09, chip 16 radius 4 0.93, 8 1.00
+// and 10 1.12, chip 24 from 1.13 up; three turned Float32 chips (sums afresh for every angle) chip 8 radius 12
+// 0.94 and 16 1.15, chip 16 radius 8 0.95 and 10 1.12, chip 24 from 1.08 up; turned integer chips (sums once)
+// chip 4 radius 4 0.96 and 5 1.02, chip 12 radius 4 0.97 and 5 1.05, chip 16 from 1.07 up.
+bool corr_fp_pays(const PassGeometry& g, bool rot, bool integer) {
+    const int64_t chip = g.max_ch * g.max_cw, surface = g.max_nr * g.max_nc;
+    if (rot && integer) return surface >= 100 || chip >= 256;
+    return 3 * chip + surface >= (rot ? 1100 : 960);
+}
+
 int ilog2_exact(int up) {
     int L = 0;
     while ((1 << L) < up) ++L;
@@ -5275,7 +5288,7 @@ cudaError_t launch_track_impl(int dtype, const void* ref, const void* sec, const
     CorrPlan P{};
     // One-tile surfaces with an FP32 numerator take k_corr_fp: turned chips (but not with a
     // diagnostic surface, which k_corr keeps across angles) and the types other than UInt8.
-    const bool fp = (rotating ? !surf_out : dtype != AR_U8) && 
+    const bool fp = (rotating ? !surf_out : dtype != AR_U8) && corr_fp_pays(geom, rotating, dtype != AR_F32) &&
                     plan_corr_fp(geom, 220 * 1024, rotating, dtype != AR_F32, &P);
     if (!fp && !plan_corr(geom, ph_bytes, 220 * 1024, &P, rotating)) {
         if (err) *err = rotating ? "chip and search geometry too large for shared memory with "
