@@ -3828,12 +3828,17 @@ __global__ void __launch_bounds__(kBfThreads, 1) k_corr_bf(const BfArgs A) {
                     if (i0 >= i1) continue;
                     const float* col = s_raw + x * A.RS;
                     double h1 = 0.0, h2 = 0.0;
+                    int nz = 0;  // Float32: values other than zero
                     for (int a = i0; a < i0 + ch; ++a) {
                         const double w = static_cast<double>(col[a]);
                         h1 = __dadd_rn(h1, w);
                         h2 = __dadd_rn(h2, __dmul_rn(w, w));
+                        if (!Tr::integer) nz += w != 0.0;
                     }
                     for (int i = i0; i < i1; ++i) {
+                        // A column of zeros sums to zero, which sliding sums of Float32 values may miss
+                        // by a rounding; the running sum along the row then stays as it is.
+                        if (!Tr::integer && nz == 0 && h2 == h2) h1 = h2 = 0.0;
                         s_V[2 * (x * A.VS + i)] = h1;
                         s_V[2 * (x * A.VS + i) + 1] = h2;
                         if (i + 1 < i1) {
@@ -3841,6 +3846,7 @@ __global__ void __launch_bounds__(kBfThreads, 1) k_corr_bf(const BfArgs A) {
                             const double wn = static_cast<double>(col[i + ch]);
                             h1 = __dadd_rn(__dsub_rn(h1, wo), wn);
                             h2 = __dadd_rn(__dsub_rn(h2, __dmul_rn(wo, wo)), __dmul_rn(wn, wn));
+                            if (!Tr::integer) nz += (wn != 0.0) - (wo != 0.0);
                         }
                     }
                 }
