@@ -5336,8 +5336,9 @@ cudaError_t launch_track_impl(int dtype, const void* ref, const void* sec, const
     const size_t ph_bytes = dtype == AR_U8 && !rotating ? 4 : 8;
     CorrPlan P{};
     // One-tile surfaces with an FP32 numerator take k_corr_fp: turned chips (but not with a
-    // diagnostic surface, which k_corr keeps across angles) and the types other than UInt8.
-    const bool fp = (rotating ? !surf_out : dtype != AR_U8) && corr_fp_pays(geom, rotating, dtype != AR_F32) &&
+    // diagnostic surface, which k_corr keeps across angles) and the types other than UInt8 (surfaces of
+    // more than one point, at max_nr rows each, are k_corr's: k_corr_fp's have a row more).
+    const bool fp = (rotating ? !surf_out : dtype != AR_U8 && (!surf_out || pts.n == 1)) && corr_fp_pays(geom, rotating, dtype != AR_F32) &&
                     plan_corr_fp(geom, 220 * 1024, rotating, dtype != AR_F32, &P);
     if (!fp && !plan_corr(geom, ph_bytes, 220 * 1024, &P, rotating)) {
         if (err) *err = rotating ? "chip and search geometry too large for shared memory with "
