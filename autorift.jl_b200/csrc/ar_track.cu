@@ -687,8 +687,9 @@ __device__ unsigned long long g_tc_phase[16];
 
 // ----------------------------------------------------------------------------------------------
 // Direct FP32 correlation of UInt16, Int16 and Float32 imagery and of turned chips of any type,
-// surfaces of one tile (k_corr_fp). The same numerator as k_corr, product for product: FP32 over
-// two chip columns in the same order, then FP64; but
+// surfaces of one tile (k_corr_fp). The numerator of k_corr: the same FP32 sums of two chip columns'
+// products, added in FP64 (in the same order, or part by part where the chip's columns are split over
+// threads: then within a few FP64 roundings); but
 //  * two surface columns per thread as packed FP32 pairs: the window is staged as pairs
 //    (W[r, x], W[r, x + 1]), so one 64-bit load feeds a packed FMA whatever the row, and a product
 //    pair costs one issue slot;
@@ -702,7 +703,9 @@ __device__ unsigned long long g_tc_phase[16];
 //    each point's variance terms are kept (8 bytes a value), not its sums, and serve every angle of
 //    an integer image;
 //  * Float32 estimates of the surface, with the FP64 normalisation (src/correlate.jl:591-600) for
-//    the candidates of the maximum and the patch only.
+//    the candidates of the maximum and the patch only;
+//  * NaN and infinite pixels of Float32 imagery show in the column sums, and such windows take a second
+//    pass over them (fp_nonfinite).
 // Bound: the FMA pipe takes two cycles for a packed warp instruction, 20.5 k cycles a point at chip
 // 32 / radius 25 of the 46 k a point takes (30 k of products per CTA without a neighbour; the box
 // sums, the window and the estimates around them are FP64 and load latency, which the other of
@@ -747,26 +750,66 @@ __device__ __noinline__ float fp_exact(double num, double wvar, double cnorm) {
     return den > 0.0 ? __double2float_rn(__ddiv_rn(num, den)) : 0.0f;
 }
 
-// The variance terms that NaN and infinite pixels of a Float32 window reach, as in k_corr's tables: an
+// The variance terms of a Float32 window with NaN or infinite pixels, as k_corr's tables have them: an
 // FP64 sum that took in a NaN, or let an infinity go, is a NaN from there on. So such a pixel reaches
-// every later row of its tile and every later column of its run of sixteen, and a variance that is
-// not a number counts as none (the value is 0). The other terms were summed with these pixels as zero.
-// `first` holds two rows a window column: the first with a NaN, the first with an infinity. Against
-// such windows left to sums that start afresh more often (other peaks than k_corr's beside a gap), this
-// costs windows without gaps 0.3 % at chip 32, radius 25 and 1.5 % at chip 16, radius 10 (the second copy of
-// the sums in the kernel; out of line 0.1 and 0.8 %, but 6 % behind k_corr over gaps).
+// every later row of its tile and every later column of its run of sixteen, and a variance that is not
+// a number counts as none (the value is 0); the other terms take these pixels as zero. A thread a column, and
+// out of line: few windows need it, and a second copy of the kernel's own sums cost the others more (8800 points
+// at chip 16, radius 10: 593 us without the check, 603 with a copy, 598 so; over one NaN in 10 000 pixels
+// 3.2 and 3.5 ms for 13 924 points of chip 32, radius 25, 4.1 with k_corr). `v` holds the column sums of four rows, then two rows a
+// window column: the first with a NaN, the first with an infinity.
 __device__ __noinline__ void fp_nonfinite(const float2* win, int XH, int WS, int ch, int cw, int nr, int nc,
-                                          int TI, int TJ, bool ncc, double* wv, int NRS, int* first) {
-    const int tid = threadIdx.x;  // at least as many as window columns
+                                          double shift, bool zncc, int TI, int TJ, double* v, double* wv, int NRS) {
+    const int tid = threadIdx.x, XW = cw + nc - 1;  // at least as many threads as window columns
+    const double nn = static_cast<double>(ch * cw);
+    double* v2 = v + 4 * kCorrThreads;
     const float2* col = win + ((tid & 1) * XH + (tid >> 1)) * WS;
+    auto value = [&](int r) {
+        const float w = col[r].x;
+        return fabsf(w) <= FLT_MAX ? __dadd_rn(static_cast<double>(w), shift) : 0.0;
+    };
+    double h1 = 0.0, h2 = 0.0;
+    int nz = 0;  // values other than zero
+    if (tid < XW)
+        for (int r = 0; r < ch; ++r) {
+            const double w = value(r);
+            h1 += w;
+            h2 += w * w;
+            nz += w != 0.0;
+        }
+    for (int i0 = 0; i0 < nr; i0 += 4) {
+        const int ni = min(4, nr - i0);
+        for (int i = 0; i < ni && tid < XW; ++i) {
+            v[i * kCorrThreads + tid] = nz ? h1 : 0.0;
+            v2[i * kCorrThreads + tid] = nz ? h2 : 0.0;
+            if (i0 + i + 1 == nr) break;  // no row below the window's last
+            const double wo = value(i0 + i), wn = value(i0 + i + ch);
+            h1 += wn - wo;
+            h2 += wn * wn - wo * wo;
+            nz += (wn != 0.0) - (wo != 0.0);
+        }
+        __syncthreads();
+        for (int t = tid; t < ni * nc; t += kCorrThreads) {
+            const int i = t / nc, j = t - i * nc;
+            double s1 = 0.0, s2 = 0.0;
+            for (int b = 0; b < cw; ++b) {
+                s1 += v[i * kCorrThreads + j + b];
+                s2 += v2[i * kCorrThreads + j + b];
+            }
+            const double var = zncc ? __dsub_rn(s2, __ddiv_rn(__dmul_rn(s1, s1), nn)) : s2;
+            wv[j * NRS + i0 + i] = var > 0.0 ? var : 0.0;
+        }
+        __syncthreads();
+    }
+    int* first = reinterpret_cast<int*>(v);
     for (int ti = 0; ti < nr; ti += TI) {
         const int te = min(ti + TI, nr), none = te + ch;
-        if (tid < cw + nc - 1) {
+        if (tid < XW) {
             int rn = none, ri = none;
             for (int r = ti; r < te + ch - 1 && rn == none; ++r) {
-                const float v = fabsf(col[r].x);
-                if (isnan(v)) rn = r;
-                else if (!(v <= FLT_MAX)) ri = min(ri, r);
+                const float w = fabsf(col[r].x);
+                if (isnan(w)) rn = r;
+                else if (!(w <= FLT_MAX)) ri = min(ri, r);
             }
             first[2 * tid] = rn;
             first[2 * tid + 1] = ri;
@@ -781,7 +824,7 @@ __device__ __noinline__ void fp_nonfinite(const float2* win, int XH, int WS, int
             }
             const int rb = min(rn, ri);
             for (int i = max(ti, rb - ch + 1); i < te; ++i)
-                wv[tid * NRS + i] = ncc && i <= rb && i + ch <= rn ? INFINITY : 0.0;
+                wv[tid * NRS + i] = !zncc && i <= rb && i + ch <= rn ? INFINITY : 0.0;
         }
         __syncthreads();
     }
@@ -1039,10 +1082,7 @@ __global__ void __launch_bounds__(kCorrThreads, 2) k_corr_fp(const CorrArgs A) {
             // surface rows; A.TI rows of each segment at a time go to shared memory, where a task
             // sums cw columns for five neighbouring values. The counts of non-zero values keep
             // windows of zeros at exactly zero, which sliding FP64 sums would miss by a rounding.
-            // kGaps: a Float32 window with pixels that are not finite, which count as zero.
-            bool nonfinite = false;  // a column sum of this thread took one in
-            auto box_sums = [&](auto gaps) {
-                constexpr bool kGaps = decltype(gaps)::value;
+            if (!have_var) {
                 const int nseg = max(1, min(8, kCorrThreads / XW));
                 const int seglen = (nr + nseg - 1) / nseg;
                 const int seg = tid / XW, x = tid - seg * XW;
@@ -1055,7 +1095,6 @@ __global__ void __launch_bounds__(kCorrThreads, 2) k_corr_fp(const CorrArgs A) {
                     if constexpr (Tr::integer) {
                         return static_cast<BS>(__float_as_int(__fadd_rn(__fadd_rn(v, cs), 12582912.0f)) - 0x4B400000);
                     } else {
-                        if (kGaps && !(fabsf(v) <= FLT_MAX)) return 0.0;
                         return __dadd_rn(static_cast<double>(v), cshift);
                     }
                 };
@@ -1168,16 +1207,10 @@ __global__ void __launch_bounds__(kCorrThreads, 2) k_corr_fp(const CorrArgs A) {
                     __syncthreads();
                 }
                 // From a pixel that is not finite on, its column's sums are not either.
-                if constexpr (!Tr::integer && !kGaps) nonfinite = !(h2 <= DBL_MAX);
-            };
-            if (!have_var) {
-                box_sums(std::false_type{});
                 if constexpr (!Tr::integer) {
-                    if (__syncthreads_or(nonfinite)) {
-                        box_sums(std::true_type{});
-                        fp_nonfinite(s_win, XH, A.WS, ch, cw, nr, nc, A.GTI, A.GTJ, A.measure == AR_NCC, s_wv,
-                                     A.NRS, reinterpret_cast<int*>(s_v1));
-                    }
+                    if (__syncthreads_or(!(h2 <= DBL_MAX)))
+                        fp_nonfinite(s_win, XH, A.WS, ch, cw, nr, nc, cshift, A.measure != AR_NCC, A.GTI, A.GTJ,
+                                     s_v1, s_wv, A.NRS);
                 }
                 have_var = Tr::integer;  // Float32 image values carry the shift's rounding
             }
@@ -2843,7 +2876,7 @@ __global__ void __launch_bounds__(kTc2Threads, 2) k_corr_tc2(const TcArgs A) {
     clear_acc();
     int dirty_ch = 0;
     // This thread's row of the chip operand and its first chip column (the same for every point).
-    const int e_groups = kTcThreads / A.NB;  // 0: more rows than threads
+    const int e_groups = kTcThreads / A.NB;  // at least one: the plan holds NB to 256
     const int e_row = tid % A.NB, e_grp = tid / A.NB;
     TC_PHASE_INIT
     // Whether s_S1, s_S2 and s_R hold the previous point's box sums, as rings of NRS rows per
