@@ -188,8 +188,8 @@ class Context:
         return a.value, b.value, t.value, n.value, f.value
 
     def tuned(self):
-        """The autotuner's choices so far: one dict per pass geometry (largest chip rows and
-        columns, surface rows and columns) with the kernel kept ("k_corr_tc2", "k_corr_tc" or
+        """The large UInt8 passes met so far: one dict per pass geometry (largest chip rows and
+        columns, surface rows and columns) with the kernel that runs it ("k_corr_tc2", "k_corr_tc" or
         "k_corr")."""
         cnt = _i64()
         self.check(self.lib.ar_ctx_tuned(self.handle, None, 0, ctypes.byref(cnt)))

@@ -437,7 +437,8 @@ __global__ void __launch_bounds__(kHpThreads) k_highpass_int(const T* img, const
 // are a sliding sum over a register ring of the last W columns. A warp writes the 32 - (W - 1)
 // rows whose whole window it holds. Bound: issue slots, not memory: with 64-bit sums and
 // addresses and the conversion unit a 6001 x 5003 UInt16 image at width 5 took 151 us, with 32-bit ones
-// 125; more warps an SM gave nothing. The mean is an FP32 division of the exact sum by the count: both are exact in FP32
+// 125; more warps an SM gave nothing. The mean is the FP32 quotient of the exact sum by the count (a
+// division, or for whole windows a product with the reciprocal and one correction): both are exact in FP32
 // (below 2^24) and FP64 has more than 2 x 24 + 2 bits, so it equals the generic kernel's FP64
 // quotient rounded to FP32 (double rounding is innocuous there); the output is the generic
 // kernel's, bit for bit.
