@@ -668,7 +668,7 @@ def rotation_measure(ar, ctx, raw, opts, grid, args, dev, stream, flush, fp32_pe
             "kernel_ms_per_pass": {"k_corr": r["k_corr_ms"], "k_refine": r["k_refine_ms"]},
             "plain_points_per_s": res["plain"]["points_per_s"],
             "cost_vs_plain": res["plain"]["points_per_s"] / r["points_per_s"],
-            "roofline": {"bound": "fp32", "kernel": "k_corr (rotation instantiation)",
+            "roofline": {"bound": "fp32", "kernel": "k_corr_fp (rotation search)",
                          "achieved": r["corr_tflops"], "peak": fp32_peak, "unit": "TFLOP/s",
                          "frac": r["corr_tflops"] / fp32_peak if (r["corr_tflops"] and fp32_peak)
                          else None,
@@ -761,9 +761,8 @@ def batching_measure(ar, ctx, torch, dev, a, b, valid, fdown, stream, flush, arg
     """The batching configuration on the benchmark pair: chip sizes 16/32/64/128 through the
     multichip search over ~1.9 M jittered centres on an 8 px lattice with per-point radii
     U[4, 48] (floored to 6 by sanitize!) and integer priors from the 4x-downsampled imposed
-    field +-3 px. Timed two ways on the device -- shape-binned passes with the autotuned kernel
-    choice (the default) and one launch per pass planned for its largest surface with the
-    default kernel rule -- with bit-identical results required."""
+    field +-3 px. Timed two ways on the device -- shape-binned passes (the default) and one launch
+    per pass planned for its largest surface -- with bit-identical results required."""
     L = ar._lib
     n = a.shape[0]
     X, Y, r, dx0, dy0 = ar.synthetic.batching_points(n, fdown[0], fdown[1])
@@ -774,21 +773,19 @@ def batching_measure(ar, ctx, torch, dev, a, b, valid, fdown, stream, flush, arg
     out = {}
     res = {}
     steps = max(3, args.steps // 4)
-    for name, bins, tune in (("binned_autotuned", 1, 1), ("one_launch_per_pass", 0, 0)):
+    for name, bins in (("shape_binned", 1), ("one_launch_per_pass", 0)):
         ctx.set_option(L.AR_OPT_SHAPE_BINS, bins)
-        ctx.set_option(L.AR_OPT_AUTOTUNE, tune)
         t = timed_steps(torch, step, stream, flush, steps, args.warmup)
         out[name] = {"points_per_s": step.n * steps / (t * 1e-3), "ms_per_step": t / steps}
         res[name] = [o.cpu().numpy() for o in step.outs] + [step.ochip.cpu().numpy()]
     ctx.set_option(L.AR_OPT_SHAPE_BINS, 1)
-    ctx.set_option(L.AR_OPT_AUTOTUNE, 1)
     same = all(np.array_equal(x.view(np.uint32) if x.dtype == np.float32 else x,
                               y.view(np.uint32) if y.dtype == np.float32 else y)
-               for x, y in zip(res["binned_autotuned"], res["one_launch_per_pass"]))
-    chip = res["binned_autotuned"][3].view(np.uint16)
+               for x, y in zip(res["shape_binned"], res["one_launch_per_pass"]))
+    chip = res["shape_binned"][3].view(np.uint16)
     out.update({"points": step.n, "grid": list(step.grid.shape), "steps": steps,
                 "speedup": out["one_launch_per_pass"]["ms_per_step"] /
-                           out["binned_autotuned"]["ms_per_step"],
+                           out["shape_binned"]["ms_per_step"],
                 "bit_identical": bool(same),
                 "points_per_chip_size": {int(c): int(np.count_nonzero(chip == c))
                                          for c in np.unique(chip) if c},
@@ -1164,7 +1161,7 @@ def profile_pass_arm(args, precision):
     spacing --spacing, `--warmup` untimed passes then `--steps` timed ones; prints one line of
     timings. precision: the split-BF16 kernel's chip-64 / radius-32 pass on the highpass-filtered
     Float32 pair (quantize = :none); otherwise the fine chip-32 / radius-25 pass of the default
-    pipeline on the prepared UInt8 pair with the autotuner off (k_corr_tc2). --chip / --radius
+    pipeline on the prepared UInt8 pair (k_corr_tc2). --chip / --radius
     replace the pass's chip size and radius (a radius above 32 runs k_corr_tc); --kernel picks
     the UInt8 kernel."""
     import torch
@@ -1292,12 +1289,12 @@ def main():
     ap.add_argument("--size", type=int, default=N,
                     help="image side; the benchmark line uses 10980, profiles a smaller scene")
     ap.add_argument("--profile", action="store_true",
-                    help="time the device steps only, autotuner off (for ncu captures); no JSON "
+                    help="time the device steps only (for ncu captures); no JSON "
                          "bench line")
     ap.add_argument("--profile-precision", action="store_true",
                     help="time the chip-64 split-BF16 track pass only (for ncu captures)")
     ap.add_argument("--profile-pass", action="store_true",
-                    help="time the fine chip-32 UInt8 track pass only, autotuner off "
+                    help="time the fine chip-32 UInt8 track pass only "
                          "(k_corr_tc2; for ncu captures)")
     ap.add_argument("--spacing", type=int, default=SPACING,
                     help="grid spacing of a --profile run (the benchmark line always uses 8)")
