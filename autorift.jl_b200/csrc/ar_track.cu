@@ -4292,6 +4292,7 @@ __global__ void __launch_bounds__(kBfThreads, 1) k_corr_bf(const BfArgs A) {
 // 10980 x 10980 scene 27.7 ms before (all three levels materialised, then a block search).
 
 constexpr int kRefineWarps = 8;
+constexpr int kRefineSplit = 4;      // warps to a patch in passes of few patches
 constexpr int kZT = 6;               // level cells per tile side
 constexpr int kZR = 2 * (kZT + 2);   // side of a stored region (rows, and its leading dimension)
 constexpr int kZC = kZT + 4;         // source columns of a tile's vertical pass
@@ -4384,8 +4385,13 @@ __device__ __forceinline__ void zoom_step(const Region& S, int n, int lo_r, int 
     __syncwarp();
 }
 
+// SPLIT: the warps of a block (kRefineSplit) search one patch. They do the same until a level's box has
+// more than one tile, which they then deal out, and the block takes the best of what they found.
+template <bool SPLIT>
 __global__ void __launch_bounds__(kRefineWarps * 32, 4) k_refine(const RefineArgs A) {
     extern __shared__ __align__(16) float rsm[];
+    __shared__ float s_best[kRefineSplit], s_v0[kRefineSplit];
+    __shared__ int s_at[kRefineSplit];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const int L = A.levels;
     // Per warp: the patch (5 columns), the vertical pass of a tile, a region for each level
@@ -4396,8 +4402,8 @@ __global__ void __launch_bounds__(kRefineWarps * 32, 4) k_refine(const RefineArg
     int* stk = reinterpret_cast<int*>(reg + (L - 1) * kZR * kZR);
     const int nfinal = 5 << L;
     const int64_t count = A.count ? static_cast<int64_t>(*A.count) : A.n_items;
-    const int64_t step = static_cast<int64_t>(gridDim.x) * warps;
-    int64_t item = static_cast<int64_t>(blockIdx.x) * warps + warp;
+    const int64_t step = SPLIT ? gridDim.x : static_cast<int64_t>(gridDim.x) * warps;
+    int64_t item = SPLIT ? blockIdx.x : static_cast<int64_t>(blockIdx.x) * warps + warp;
     float next = item < count && lane < 25 ? A.patch[item * 25 + lane] : 0.0f;
     for (; item < count; item += step) {
         const float pv = next;
@@ -4420,6 +4426,7 @@ __global__ void __launch_bounds__(kRefineWarps * 32, 4) k_refine(const RefineArg
         Region S{P0, 0, 0};
         Window box{0, 4, 0, 4};
         int tile = 0, ntr = 1, ntc = 1;
+        int dealt = -1;      // SPLIT: the level whose tiles are dealt out
         if (zeros) bv = v0 = 0.0f, bi = 0;
         while (!zeros) {
             const int n = 5 << l;
@@ -4431,7 +4438,7 @@ __global__ void __launch_bounds__(kRefineWarps * 32, 4) k_refine(const RefineArg
                 t.c = box.c + (tile / ntr) * kZT;
                 t.d = min(t.c + kZT, box.d);
             }
-            ++tile;
+            tile += SPLIT && l == dealt ? kRefineSplit : 1;
             const float e_l = ldexpf(esum, 2 - 2 * l) + slack;
             bool skip = false;
             if (ntr * ntc > 1) {
@@ -4550,6 +4557,11 @@ __global__ void __launch_bounds__(kRefineWarps * 32, 4) k_refine(const RefineArg
                         tile = 0;
                         ntr = max(1, (k.b - k.a + kZT - 1) / kZT);
                         ntc = max(1, (k.d - k.c + kZT - 1) / kZT);
+                        if (SPLIT && dealt < 0 && ntr * ntc > 1) {
+                            dealt = l;
+                            tile = warp;
+                            if (tile >= ntr * ntc) break;  // none for this warp (and no other level pending)
+                        }
                     } else {
                         descend = false;
                     }
@@ -4574,7 +4586,20 @@ __global__ void __launch_bounds__(kRefineWarps * 32, 4) k_refine(const RefineArg
         } else {
             v0 = __shfl_sync(kFull, v0, 0);  // lane 0 computes sample (0, 0)
         }
-        if (lane == 0) {
+        if constexpr (SPLIT) {
+            if (lane == 0) {
+                s_best[warp] = bv;
+                s_at[warp] = bi;
+                s_v0[warp] = v0;
+            }
+            __syncthreads();
+            for (int w = 0; w < kRefineSplit; ++w) {
+                best_update(s_best[w], s_at[w], bv, bi);
+                v0 = isnan(v0) ? s_v0[w] : v0;
+            }
+            __syncthreads();  // read before the next patch's
+        }
+        if (lane == 0 && (!SPLIT || warp == 0)) {
             int si = 0, sj = 0;
             float v = bv;
             if (bi != INT_MAX && bv != -INFINITY) {
@@ -4836,6 +4861,24 @@ RefinePlan plan_refine(int up) {
     R.per_sm = std::max(1, best_sm);
     R.smem = static_cast<size_t>(R.warps) * per_warp;
     return R;
+}
+
+// Refinement of at most n patches. Up to four patches an SM a block of kRefineSplit warps takes each: the
+// call then waits for its slowest patch, and one whose box does not shrink (noise, ties) visits many tiles.
+// Noise, us a call of bare patches with a warp each and split: 50 at 16x 77 and 66, at 64x 92 and 78, 592 at
+// 16x 83 and 68; smooth peaks 592 at 16x 59 and 61, 1184 65 and 75.
+cudaError_t launch_refine(const RefinePlan& R, const RefineArgs& B, int64_t n, int num_sms, cudaStream_t stream) {
+    const bool split = n <= 4 * static_cast<int64_t>(num_sms);
+    const int warps = split ? kRefineSplit : R.warps;
+    const size_t smem = static_cast<size_t>(warps) * R.warp_floats * sizeof(float);
+    if (smem > static_cast<size_t>(kDynSmemCap)) return cudaErrorInvalidValue;
+    auto kern = split ? k_refine<true> : k_refine<false>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kDynSmemCap);
+    if (e != cudaSuccess) return e;
+    const int64_t blocks = split ? n : std::min<int64_t>((n + R.warps - 1) / R.warps,
+                                                         static_cast<int64_t>(num_sms) * R.per_sm);
+    kern<<<static_cast<unsigned>(std::max<int64_t>(1, blocks)), warps * 32, smem, stream>>>(B);
+    return cudaGetLastError();
 }
 
 // Dynamic shared memory a CTA holding `cols` Tensor Memory columns reserves, for a kernel with
@@ -5657,14 +5700,8 @@ cudaError_t launch_track_impl(int dtype, const void* ref, const void* sec, const
     B.out = out;
     B.levels = R.levels;
     B.warp_floats = R.warp_floats;
-    if (R.smem > static_cast<size_t>(kDynSmemCap)) return cudaErrorInvalidValue;
-    e = cudaFuncSetAttribute(k_refine, cudaFuncAttributeMaxDynamicSharedMemorySize, kDynSmemCap);
+    e = launch_refine(R, B, pts.n, num_sms, stream);
     if (e != cudaSuccess) return e;
-    const int rgrid = static_cast<int>(std::max<int64_t>(
-        1, std::min<int64_t>((pts.n + R.warps - 1) / R.warps,
-                             static_cast<int64_t>(num_sms) * R.per_sm)));
-    k_refine<<<rgrid, R.warps * 32, R.smem, stream>>>(B);
-    e = cudaGetLastError();
     T.launches += 1;
     if (T.enabled) {
         cudaEventRecord(ev2, stream);
@@ -5701,15 +5738,7 @@ cudaError_t launch_refine_patches(const float* patches, int64_t count, int up, i
     B.oval = value;
     B.levels = R.levels;
     B.warp_floats = R.warp_floats;
-    if (R.smem > static_cast<size_t>(kDynSmemCap)) return cudaErrorInvalidValue;
-    cudaError_t e =
-        cudaFuncSetAttribute(k_refine, cudaFuncAttributeMaxDynamicSharedMemorySize, kDynSmemCap);
-    if (e != cudaSuccess) return e;
-    const int grid = static_cast<int>(std::max<int64_t>(
-        1, std::min<int64_t>((count + R.warps - 1) / R.warps,
-                             static_cast<int64_t>(num_sms) * R.per_sm)));
-    k_refine<<<grid, R.warps * 32, R.smem, stream>>>(B);
-    return cudaGetLastError();
+    return launch_refine(R, B, count, num_sms, stream);
 }
 
 }  // namespace ar

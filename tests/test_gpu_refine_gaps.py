@@ -1,4 +1,4 @@
-"""k_refine on patches with NaN and on patches of zeros, against the full Float32 cascade: identical value and
+"""k_refine on patches with NaN, of zeros and of noise, against the full Float32 cascade: identical value and
 row-major-first position at every factor. NaN at each of the 25 places, whole rows and columns of them,
 few values left, beside smooth peaks, rough and tied values; zeros of either sign."""
 
@@ -36,6 +36,9 @@ def patches(kind, rng):
                 p[:, rng.integers(5)] = np.nan
             out.append(p)
         out.append(np.full((5, 5), np.nan))
+    elif kind == "rough":  # boxes that do not shrink; infinite and huge values
+        out = [rng.standard_normal((5, 5)) for _ in range(40)]
+        out += [np.where(rng.random((5, 5)) < 0.1, bad, base(1)) for bad in (np.inf, -np.inf, 3e38)]
     else:
         out = [np.zeros((5, 5)), -np.zeros((5, 5)), np.where((i + j) % 2, 0.0, -0.0)]
         out += [np.where((i == r) & (j == c), v, 0.0) for r, c in ((0, 0), (2, 2), (4, 4), (0, 3)) for v in (1e-45, -1.0)]
@@ -43,10 +46,13 @@ def patches(kind, rng):
 
 
 @pytest.mark.parametrize("up", [2, 4, 8, 16, 64, 128])
-@pytest.mark.parametrize("kind", ["one", "many", "zeros"])
-def test_matches_cascade(ar, gpu_lib, up, kind):
+@pytest.mark.parametrize("kind", ["one", "many", "zeros", "rough"])
+@pytest.mark.parametrize("count", [1, 2, 592, 593])
+def test_matches_cascade(ar, gpu_lib, up, kind, count):
+    """Up to 592 patches a block of four warps takes each, beyond a warp does."""
     P = patches(kind, np.random.default_rng(up))
-    row, col, val = ar.refine_patches(P, up)
+    row, col, val = (v.reshape(-1) for v in ar.refine_patches(np.resize(P, (count, 5, 5)), up))
+    P = P[:count]
     with np.errstate(all="ignore"):
         for k, p in enumerate(P):
             s = p
