@@ -3686,7 +3686,6 @@ __global__ void __launch_bounds__(kBfThreads, 1) k_corr_bf(const BfArgs A) {
     extern __shared__ __align__(1024) unsigned char smem_bf[];
     __shared__ uint64_t s_mbar[2];
     __shared__ uint32_t s_taddr;
-    __shared__ int s_slot;
     const int tid = threadIdx.x, bd = blockDim.x;
     const int lane = tid & 31, warp = tid >> 5;
     const T* ref = static_cast<const T*>(A.ref);
@@ -4185,9 +4184,6 @@ __global__ void __launch_bounds__(kBfThreads, 1) k_corr_bf(const BfArgs A) {
             failed = true;
             break;
         }
-        // The products are here and nothing below gives up, so the patch of this slot of the
-        // refinement queue will be written (k_refine trusts the count).
-        if (tid == 0 && !(A.up == 1 || nr < 5 || nc < 5)) s_slot = atomicAdd(A.sub_count, 1);
 
         // Epilogue: every value normalised in FP64 into the surface in shared memory.
         {
@@ -4239,15 +4235,21 @@ __global__ void __launch_bounds__(kBfThreads, 1) k_corr_bf(const BfArgs A) {
         } else {
             const int pi0 = min(max(pi - 2, 0), max(nr - 5, 0));
             const int pj0 = min(max(pj - 2, 0), max(nc - 5, 0));
-            const int slot = s_slot;
-            if (tid < 25) {
-                const int a = tid % 5, b = tid / 5;
-                A.sub_patch[static_cast<int64_t>(slot) * 25 + tid] = s_surf[(pj0 + b) * A.NRS + (pi0 + a)];
-            }
-            if (tid == 0) {
-                A.sub_point[slot] = k;
-                A.sub_origin[2 * slot] = pi0;
-                A.sub_origin[2 * slot + 1] = pj0;
+            // The products were here and nothing gave up: the slot of the refinement queue that is taken now
+            // is written (k_refine trusts the count).
+            if (warp == 0) {
+                int slot = 0;
+                if (lane == 0) slot = atomicAdd(A.sub_count, 1);
+                slot = __shfl_sync(kFull, slot, 0);
+                if (lane < 25) {
+                    const int a = lane % 5, b = lane / 5;
+                    A.sub_patch[static_cast<int64_t>(slot) * 25 + lane] = s_surf[(pj0 + b) * A.NRS + (pi0 + a)];
+                }
+                if (lane == 0) {
+                    A.sub_point[slot] = k;
+                    A.sub_origin[2 * slot] = pi0;
+                    A.sub_origin[2 * slot + 1] = pj0;
+                }
             }
         }
         TC_PHASE(11)
